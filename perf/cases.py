@@ -155,7 +155,7 @@ def _inputs(c, seed):
         sa = (c["m"], c["k"]) if c["opA"] == "N" else (c["k"], c["m"])
         sb = (c["k"], c["n"]) if c["opB"] == "N" else (c["n"], c["k"])
         f = 1.0 / np.sqrt(c["k"])
-        return [(_cn(rng, sa, 1.0) * f, _cn(rng, sb, 1.0), _cn(rng, (c["m"], c["n"]), 1.0)) for _ in range(c["count"])]
+        return [(_cn(rng, sa, 1.0) * f, _cn(rng, sb, 1.0)) for _ in range(c["count"])]
     if k in ("rgf", "keldysh", "ddrgf"):
         sizes = _sizes(c)
         d = _device(rng, sizes)
@@ -200,6 +200,29 @@ def _block_matrix(lib, sizes, Md, Mu, Ml, hermitian=False):
     return bm
 
 
+def _arena(shapes):
+    """Column-major blocks of the given shapes in one zeroed allocation: (all of it, the blocks)."""
+    flat = torch.zeros(sum(m * n for m, n in shapes), dtype=torch.complex128, device="cuda")
+    blocks, o = [], 0
+    for m, n in shapes:
+        blocks.append(flat[o:o + m * n].view(n, m).t())
+        o += m * n
+    return flat, blocks
+
+
+def _into_arena(bm, keys):
+    """Give a BlockMatrix one allocation for all of its blocks (key order)."""
+    flat, blocks = _arena([(bm.blockSizes[i], bm.blockSizes[j]) for i, j in keys])
+    for k, b in zip(keys, blocks):
+        bm.M[k] = b
+    return flat
+
+
+def _keys(n, lower=True):
+    return sorted(p for i in range(n) for p in ((i, i), (i, i + 1), (i, i - 1))
+                  if 0 <= p[1] < n and (lower or p[1] >= p[0]))
+
+
 def prepare(c, seed):
     import libnegf_b200 as lib
 
@@ -208,21 +231,24 @@ def prepare(c, seed):
     s = dict(case=c, lib=lib)
     if k == "inv":
         s["A"] = [lib.to_device(a) for a in x]
-        s["out"] = [lib.dzeros(*a.shape) for a in x]
+        s["flat"], s["out"] = _arena([a.shape for a in x])
     elif k == "gemm":
-        s["items"] = [(1.0, lib.to_device(a), lib.to_device(b), 0.0, lib.to_device(cc)) for a, b, cc in x]
+        s["flat"], out = _arena([(c["m"], c["n"])] * len(x))
+        s["items"] = [(1.0, lib.to_device(a), lib.to_device(b), 0.0, cc) for (a, b), cc in zip(x, out)]
     elif k in ("rgf", "keldysh", "ddrgf"):
         sizes, Md, Mu, Ml, Sd, Su = x
         s["M"] = _block_matrix(lib, sizes, Md, Mu, Ml)
         if k == "rgf":
             s["out"] = lib.BlockMatrix(sizes, None, {"in": 3, "out": 3}, False, False)
-            lib.bm_blocks_define_(s["out"], 1)
+            s["flat"] = _into_arena(s["out"], _keys(len(sizes)))
             s["aux"] = lib.allocate_aux_data_RGF(s["M"])
         elif k == "keldysh":
             s["S"] = _block_matrix(lib, sizes, Sd, Su, None, True)
             s["aux"] = lib.allocate_aux_data_Keldysh(s["M"], s["S"])
+            s["flat"] = _into_arena(s["aux"].buffS, _keys(len(sizes), lower=False))
         else:
             s["aux"] = lib.allocate_aux_data_DDRGF(s["M"])
+            s["flat"] = _into_arena(s["aux"][0].buffMout, _keys(len(sizes)))
     elif k == "solver":
         devs, E = x
         dev = [lib.Device(d["Hd"], d["Hu"], d["sL"], d["sR"]) for d in devs]
@@ -257,20 +283,19 @@ def run(s):
     k = c["kind"]
     if k == "inv":
         lib.be_inv_batched_(s["A"], s["out"])
-        return list(s["out"])
+        return s["flat"]
     if k == "gemm":
         lib.be_gemm_batched_(c["opA"], c["opB"], s["items"], c["precision"])
-        return [it[4] for it in s["items"]]
+        return s["flat"]
     if k == "rgf":
         lib.bndiag_of_inv_rgf_local_(s["out"], s["M"], s["aux"])
-        return [s["out"].M[p] for p in sorted(s["out"].M)]
+        return s["flat"]
     if k == "keldysh":
         lib.keldyshndiag_(s["M"], s["S"], s["aux"])
-        return [s["aux"].buffS.M[p] for p in sorted(s["aux"].buffS.M)]
+        return s["flat"]
     if k == "ddrgf":
         lib.bndiag_of_inv_ddrgf_(s["M"], s["aux"])
-        m = s["aux"][0].buffMout.M
-        return [torch.cat([m[p].t().reshape(-1) for p in sorted(m) if p[0] - p[1] == d]) for d in (0, -1, 1)]
+        return s["flat"]
     if k == "solver":
         st = s["stream"].cuda_stream
         s["solver"].set_energies(s["E"], st)
@@ -284,7 +309,7 @@ def run(s):
             s["outs"][0].data_ptr(), s["outs"][1].data_ptr(), s["outs"][2].data_ptr(), 1, lib.stream_handle()))
         return list(s["outs"])
     gr, gl, t = s["device"].solve(s["E"], eta=ETA_E, mu_l=MU_L, mu_r=MU_R, kT=KT, precision=c["precision"])
-    return [np.stack([np.stack(r) for r in gr]), np.stack([np.stack(r) for r in gl]), t]
+    return [gr[0][0].base, gl[0][0].base, t]  # the whole arrays that the blocks are views of
 
 
 # --------------------------------------------------------------------------
@@ -384,26 +409,29 @@ def _colmajor(blocks):
     return torch.stack([x.mT for x in blocks], 1).reshape(-1)
 
 
+def _flat(blocks):
+    """The blocks one after the other, column-major."""
+    return torch.cat([torch.as_tensor(b).mT.reshape(-1) for b in blocks])
+
+
 def exact(c, seed):
     x = _inputs(c, seed)
     k = c["kind"]
     if k == "inv":
-        return [np.linalg.inv(a) for a in x]
+        return _flat([np.linalg.inv(a) for a in x])
     if k == "gemm":
         f = dict(N=lambda a: a, T=lambda a: a.T, C=lambda a: a.conj().T)
-        return [f[c["opA"]](a) @ f[c["opB"]](b) for a, b, _ in x]
+        return _flat([f[c["opA"]](a) @ f[c["opB"]](b) for a, b in x])
     if k in ("rgf", "ddrgf", "keldysh"):
         sizes, Md, Mu, Ml, Sd, Su = x
         n = len(sizes)
         Md, Mu, Ml = ([_t(a) for a in v] for v in (Md, Mu, Ml))
         d, u, l, g, R, L = _tri_inverse(Md, Mu, Ml)
-        if k == "rgf":
+        if k != "keldysh":
             got = {(i, i): d[i] for i in range(n)}
             got.update({(i, i + 1): u[i] for i in range(n - 1)})
             got.update({(i + 1, i): l[i] for i in range(n - 1)})
-            return [got[p] for p in sorted(got)]
-        if k == "ddrgf":
-            return [torch.cat([a.t().reshape(-1) for a in v]) for v in (d, u, l)]
+            return _flat([got[p] for p in _keys(n)])
         # G S G^H: up with the right-connected operator, down with G
         Sd, Su = [_t(a) for a in Sd], [_t(a) for a in Su]
         A, B = [a.clone() for a in Sd], [a.clone() for a in Su]
@@ -419,7 +447,7 @@ def exact(c, seed):
             G[i + 1] = G[i + 1] - L[i] @ U[i]
         got = {(i, i): G[i] for i in range(n)}
         got.update({(i, i + 1): U[i] for i in range(n - 1)})
-        return [got[p] for p in sorted(got)]
+        return _flat([got[p] for p in _keys(n, lower=False)])
     if k == "solver":
         devs, E = x
         gr, gl, t = [], [], []
@@ -436,4 +464,4 @@ def exact(c, seed):
         dd, u, l = _tri_inverse(Md, Mu, Ml)[:3]
         return [_colmajor(v) for v in (dd, u, l)]
     dd, gl, T = _exact_solver(d, E, False)
-    return [torch.stack(dd, 1), torch.stack(gl, 1), T]
+    return [_colmajor(dd), _colmajor(gl), T]
