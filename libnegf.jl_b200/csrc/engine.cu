@@ -493,22 +493,25 @@ void Plan::inv(const std::vector<InvSpec>& specs) {
   for (int k0 = 0; k0 < max_n; k0 += nb) {
     Step s;
     s.kind = Step::GJ_PANEL;
-    s.off = off; s.count = (int)v.size(); s.k0 = k0; s.nb = nb; s.blocked = 1;
+    s.off = off; s.count = (int)v.size(); s.k0 = k0; s.nb = nb; s.blocked = gj_update_int8() ? 2 : 1;
     s.smem = zgj_panel_smem_bytes(max_n, nb);
     s.max_n = max_n;
     steps.push_back(s);
+    if (!gj_update_int8()) {
+      s.kind = Step::GEMM;
+      s.form = 4;
+      for (const auto& p : v) s.flops += 8.0 * p.n * (double)p.n * std::max(0, std::min(nb, p.n - k0));
+      steps.push_back(s);
+      continue;
+    }
     std::vector<ZGemmProblem> g;
     for (const auto& p : v) {
       if (p.n <= k0) continue;
       int w = std::min(nb, p.n - k0);
       g.push_back(gp(p.F, p.n, p.Bbuf, w, p.W, p.ld, p.n, p.n, w, ONE, p.W, p.ld, ONE));
     }
-    // W += F Bbuf: INT8 digit products at FP64 accuracy in a mixed plan (the
-    // panels stay in FP64), else DMMA
-    if (gj_update_int8())
-      gemm_mixed('N', 'N', g, 34);
-    else
-      gemm_fp64('N', 'N', g);
+    // W += F Bbuf as INT8 digit products at FP64 accuracy (the panels stay in FP64)
+    gemm_mixed('N', 'N', g, 34);
   }
   // the GEMM updates carry their own flop count; the panel work is the rest
   Step u;
@@ -644,7 +647,7 @@ cudaError_t Plan::finalize() {
   std::set<std::pair<char, char>> ops;
   size_t max_smem = 0, lu_smem = 0, tri_smem = 0;
   for (const auto& s : steps) {
-    if (s.kind == Step::GEMM) ops.insert({s.opA, s.opB});
+    if (s.kind == Step::GEMM && s.form != 4) ops.insert({s.opA, s.opB});
     if (s.kind == Step::GJ_PANEL) max_smem = std::max(max_smem, s.smem);
     if (s.kind == Step::LU_PANEL) lu_smem = std::max(lu_smem, s.smem);
     if (s.kind == Step::TRI_DIAG) tri_smem = std::max(tri_smem, s.smem);
@@ -753,6 +756,10 @@ cudaError_t Plan::launch_step(const Step& s, const unsigned char* base, cudaStre
   {
     switch (s.kind) {
       case Step::GEMM:
+        if (s.form == 4) {
+          e = launch_zgj_update(reinterpret_cast<const ZInvProblem*>(base + s.off), s.count, s.k0, s.nb, s.max_n, stream);
+          break;
+        }
         e = launch_zgemm_batched_ex(s.opA, s.opB, s.preload, reinterpret_cast<const ZGemmProblem*>(base + s.off),
                                     reinterpret_cast<const int*>(base + s.tiles_off), s.count, s.total_tiles, stream, s.form,
                                     s.uniform_tiles);

@@ -35,10 +35,11 @@ int zgemm_tiles_smallk(int m, int n);
 size_t zgemm_smem_bytes();
 cudaError_t zgemm_prepare(char opA, char opB);
 size_t zgj_panel_smem_bytes(int n, int nb);
-// max_n (the largest block of the batch) selects the register-resident panel
-// kernel where it applies; 0 keeps the shared-memory one
+// max_n: the largest block of the batch (the thread count and rows per thread follow it)
 cudaError_t launch_zgj_panel(const ZInvProblem* probs_dev, int nprob, int k0, int nb, int blocked, size_t smem,
-                             cudaStream_t stream, int max_n = 0);
+                             cudaStream_t stream, int max_n);
+// rank-nb update of the panel at k0 (panel launched with blocked = 1)
+cudaError_t launch_zgj_update(const ZInvProblem* probs_dev, int nprob, int k0, int nb, int max_n, cudaStream_t stream);
 cudaError_t launch_zgj_unpermute(const ZInvProblem* probs_dev, int nprob, int max_n, cudaStream_t stream);
 cudaError_t launch_zblockops(const ZBlockOp* ops_dev, int nops, int max_m, int max_n, cudaStream_t stream);
 cudaError_t launch_ztrace_prod(const void* probs_dev, int nprob, cudaStream_t stream);
@@ -142,7 +143,7 @@ struct Step {
   int count = 0, total_tiles = 0, max_m = 0, max_n = 0;
   int k0 = 0, nb = 0, blocked = 0;
   bool preload = false;  // GEMM: accumulators start from Cin (all problems alpha, beta = +-1)
-  int form = 0;          // GEMM: 0 default, 1 four real products, 2 3M, 3 small-K 3M; OZ_MMA: digit pairs (34 or 28)
+  int form = 0;          // GEMM: 0 default, 1 four real products, 2 3M, 3 small-K 3M, 4 Gauss-Jordan update; OZ_MMA: digit pairs (34 or 28)
   int uniform_tiles = 0; // GEMM: tiles of every problem when all have the same count, else 0
   size_t smem = 0;
   double flops = 0.0;    // real flops of the step (8mnk per complex GEMM)

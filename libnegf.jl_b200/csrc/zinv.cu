@@ -9,342 +9,448 @@
 //
 // Algorithm (per matrix, n x n, panel width nb):
 //   for each panel K = [k0, k0+nb):
-//     * panel kernel (one CTA per matrix): the n x nb slab W[:,K] is held in
-//       shared memory; for each column c: warp-level arg-max of |re|+|im| over
-//       rows not yet used as pivots (LAPACK's izamax rule, ties to the lowest
-//       row), then the in-place Gauss-Jordan step on the slab.  No rows are
-//       swapped; the pivot row of column c is recorded in piv[c].  The kernel
-//       writes the slab back and prepares the rank-nb update
-//         F = slab - E_P (E_P has 1 at (piv[k0+i], i)),  Bbuf = W[P, :] with
-//         the K columns zeroed;
-//     * a batched GEMM applies W += F * Bbuf (the same kernel as all other
-//       products).
+//     * the panel kernel (one CTA per matrix) runs the in-place Gauss-Jordan
+//       steps of the n x nb slab W[:,K] in shared memory.  No rows are swapped;
+//       the pivot row of column c is recorded in piv[c];
+//     * the update kernel applies W += slab W[P, :] to the other columns (and
+//       sets the pivot rows P to slab W[P, :]).
 //   Finally inv(X)[r, piv[c]] = W[piv[r], c]; a gather kernel writes the
 //   un-permuted inverse to its destination.
-// When n * n fits in shared memory the whole matrix is one panel and no GEMM
+// When n * n fits in shared memory the whole matrix is one panel and no update
 // is needed.
 #include "negf_common.cuh"
 
 namespace negf {
 
-constexpr int GJ_THREADS = 512;
+namespace gj {
+constexpr int SW = 8;  // columns of a sub-panel, factored in registers
+}
 
 struct GjPanelArgs {
   int k0;      // first column of this panel
   int nb;      // panel width (columns)
-  int blocked; // 1: write F/Bbuf for the trailing GEMM; 0: whole matrix in one panel
+  int blocked; // 0: whole matrix in one panel; 1: zgj_update_kernel follows; 2: write F and Bbuf for a GEMM update
 };
 
-__device__ __forceinline__ void argmax_merge(double& v, int& r, double v2, int r2) {
-  if (v2 > v || (v2 == v && r2 >= 0 && (r < 0 || r2 < r))) { v = v2; r = r2; }
+// 1/a (0 for a = 0, and for infinite a).  a is scaled by a power of two
+// (exact), so that d = |a|^2 lies within [2^-102, 32); 1/d starts from a
+// single-precision reciprocal and takes one third-order Newton-Raphson step,
+// x (1 + e + e^2) with e = 1 - d x: |e| < 2^-21, so the step's error e^3 is
+// below the FP64 rounding.  No branch and no compare on the FP64 pipe: its
+// latency is part of every column's.
+__device__ __forceinline__ cplx gj_pivot_inv(cplx a) {
+  const int hx = __double2hiint(a.x) & 0x7fffffff, hy = __double2hiint(a.y) & 0x7fffffff;
+  const int e = max(hx, hy) >> 20;
+  const double s = __hiloint2double(max(1, 2046 - e) << 20, 0);
+  const double x = a.x * s, y = a.y * s;
+  const double d = fma(x, x, y * y);
+  float xf;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(xf) : "f"((float)d));
+  const double x0 = xf;
+  const double r = fma(-d, x0, 1.0);
+  const double t = fma(x0, fma(r, r, r), x0);
+  const bool none = (hx | hy | __double2loint(a.x) | __double2loint(a.y)) == 0 || e == 0x7ff;
+  return none ? make_double2(0.0, 0.0) : make_double2(x * t * s, -y * t * s);
 }
 
-__global__ void __launch_bounds__(GJ_THREADS)
+// a - b c with four fused operations
+__device__ __forceinline__ cplx gj_cfms(cplx a, cplx b, cplx c) {
+  return make_double2(fma(b.y, c.y, fma(-b.x, c.x, a.x)), fma(-b.y, c.x, fma(-b.x, c.y, a.y)));
+}
+
+__device__ __forceinline__ void gj_cp16(cplx* smem, const cplx* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem));
+}
+// with in = false: zeros (any valid address)
+__device__ __forceinline__ void gj_cp16z(cplx* smem, const cplx* gmem, bool in, const cplx* any) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
+               "l"(in ? gmem : any), "r"(in ? 16 : 0));
+}
+__device__ __forceinline__ void gj_cp_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+__device__ __forceinline__ void gj_dmma(double (&c)[4], double a0, double a1, double b0) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a0), "d"(a1), "d"(b0));
+}
+
+// Pivot candidates compare as 32-bit keys: the leading 21 bits of |re| + |im|
+// (exponent and 10 mantissa bits; plus 1, so that 0 means no candidate) over
+// 1023 - row, so that one REDUX gives value and row.  The pivot is within 0.1 %
+// of the largest |re| + |im| of its column, the lowest row among those that
+// share the leading bits; the growth bound of partial pivoting changes by that
+// factor only.
+__device__ __forceinline__ unsigned gj_key(double v, int row) {
+  return ((((unsigned)__double2hiint(v) >> 10) + 1u) << 10) | (unsigned)(1023 - row);
+}
+
+// Gauss-Jordan on an n x w slab held in shared memory (column-major, odd
+// leading dimension ldw), one CTA per matrix, in sub-panels of SW = 8 columns:
+//  * the sub-panel is factored in registers, one row per thread (RT rows for n
+//    > T).  Per column: every thread inverts its own entry while one warp
+//    reduction (REDUX) of the keys finds the warp's pivot candidate, whose lane
+//    publishes its row divided by the pivot; one barrier; every thread merges
+//    the T/32 keys, reads the winner's row and updates its own;
+//  * W[pivot rows, other columns] is copied aside (Bb) and the other columns of
+//    the slab take the rank-8 update on the FP64 tensor path (16 x 8 tiles, k =
+//    8, four real products): W += S Bb, and W = S Bb at the pivot rows (the
+//    form W += (S - E_P) Bb would lose digits where |S| is far below 1).
+// What bounds it: the latency of a column (about 900 cycles with four warps,
+// 1200 with eight: two reduction rounds, one barrier, one reciprocal, and some
+// 250 instructions per warp) and the FP64 pipe of one SM in the rank-8 updates.
+// Eight columns keep a row in 32 registers; wider sub-panels do more of the
+// n w^2 work in the latency-bound form, narrower ones add update passes over
+// shared memory.  A 256 x 32 panel takes 44 us (104 us with the whole slab in
+// registers and one rank-1 step per column), a whole 64 x 64 inversion 63 us
+// (192 us for 64 of them before), 100 x 100 131 us (627 us).
+template <int T, int RT>
+__global__ void __launch_bounds__(T)
     zgj_panel_kernel(const ZInvProblem* __restrict__ probs, GjPanelArgs args) {
+  using gj::SW;
   const ZInvProblem p = probs[blockIdx.x];
   const int n = p.n;
   const int k0 = args.k0;
   if (n <= 0 || k0 >= n) return;
   const int w = min(args.nb, n - k0);
-  constexpr int NW = GJ_THREADS / 32;
+  constexpr int NW = T / 32;
+  const int ldw = n | 1;
+  const int wt = (w + SW - 1) / SW;  // column tiles of the slab
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx* S = reinterpret_cast<cplx*>(smem_raw);  // n x w, column-major
-  cplx* colbuf = S + (size_t)n * w;               // n
-  cplx* rowbuf = colbuf + n;                       // w
-  double* redv = reinterpret_cast<double*>(rowbuf + w);  // NW (pivot value of the column, as complex below)
-  int* redr = reinterpret_cast<int*>(redv + NW);   // NW
-  int* sh_piv = redr + NW;                          // w
-  uint8_t* used = reinterpret_cast<uint8_t*>(sh_piv + w);  // n
-  cplx* sh_pv = reinterpret_cast<cplx*>(redv);      // reuses redv[0..1]: the scaled pivot inverse
+  cplx* S = reinterpret_cast<cplx*>(smem_raw);       // ldw x 8 wt
+  cplx* Bb = S + (size_t)ldw * SW * wt;               // 8 wt columns of 8 pivot-row values
+  cplx* slot = Bb + (size_t)SW * SW * wt;             // [2][NW][SW] candidate rows
+  uint4* part = reinterpret_cast<uint4*>(slot + 2 * NW * SW);  // [2][NW] candidate keys
+  int* sh_piv = reinterpret_cast<int*>(part + 2 * NW / 4);     // w
+  uint8_t* at = reinterpret_cast<uint8_t*>(sh_piv + w);         // n: the sub-panel whose pivot row a row is
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // column-per-warp, row-per-lane loops (no integer division)
   for (int j = warp; j < w; j += NW)
-    for (int r = lane; r < n; r += 32) S[(size_t)j * n + r] = p.W[r + (size_t)(k0 + j) * p.ld];
-  for (int r = tid; r < n; r += GJ_THREADS) used[r] = (k0 == 0) ? 0 : p.used[r];
+    for (int r = lane; r < n; r += 32) gj_cp16(S + (size_t)j * ldw + r, p.W + r + (size_t)(k0 + j) * p.ld);
+  bool used[RT];
+#pragma unroll
+  for (int k = 0; k < RT; ++k) {
+    const int r = tid + k * T;
+    used[k] = r >= n || (k0 > 0 && p.used[r]);
+  }
+  for (int c = tid; c < w; c += T) sh_piv[c] = 0;  // valid row indices even if the column loop stops early
+  for (int r = tid; r < n; r += T) at[r] = 255;
+  gj_cp_wait();
   __syncthreads();
 
-  for (int c = 0; c < w; ++c) {
-    if (warp == 0) {
-      // pivot search over unused rows, then stage column c and the scaled pivot row
-      double bv = -1.0;
-      int br = -1;
-      for (int r = lane; r < n; r += 32)
-        if (!used[r]) argmax_merge(bv, br, cabs1(S[(size_t)c * n + r]), r);
+  const bool active = warp * 32 < n;  // warps without rows only take part in the barriers and the updates
+  bool dead = false;  // a column without a candidate row: the host reports the info code
+  for (int s0 = 0; s0 < w && !dead; s0 += SW) {
+    const int sw = min(SW, w - s0);
+    cplx a[RT][SW];
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        double v2 = __shfl_xor_sync(0xffffffffu, bv, off);
-        int r2 = __shfl_xor_sync(0xffffffffu, br, off);
-        argmax_merge(bv, br, v2, r2);
+    for (int k = 0; k < RT; ++k)
+#pragma unroll
+      for (int j = 0; j < SW; ++j) {
+        const int r = tid + k * T;
+        a[k][j] = (r < n && j < sw) ? S[(size_t)(s0 + j) * ldw + r] : make_double2(0.0, 0.0);
       }
-      const int pr = br;  // identical in every lane after the xor reduction
-      if (lane == 0) {
-        sh_piv[c] = pr;
-        if (pr < 0 || bv == 0.0) {
-          if (p.info) atomicCAS(p.info, 0, k0 + c + 1);
+    // candidate of the current column: this thread's key (NaN rows never qualify) and entry
+    unsigned key = 0, wkey = 0;
+    cplx cand = make_double2(0.0, 0.0);
+    auto search = [&] {
+      key = 0;
+#pragma unroll
+      for (int k = 0; k < RT; ++k) {
+        const double v = cabs1(a[k][0]);
+        const unsigned q = !used[k] && __double2hiint(v) <= 0x7ff00000 ? gj_key(v, tid + k * T) : 0u;
+        if (q > key) {
+          key = q;
+          cand = a[k][0];
         }
-        if (pr >= 0) used[pr] = 1;
       }
-      if (pr >= 0) {
-        cplx pivv = S[(size_t)c * n + pr];
-        cplx pv = (pivv.x == 0.0 && pivv.y == 0.0) ? make_double2(0.0, 0.0) : cinv(pivv);
-        for (int r = lane; r < n; r += 32) colbuf[r] = S[(size_t)c * n + r];
-        for (int j = lane; j < w; j += 32) rowbuf[j] = (j == c) ? pv : cmul(S[(size_t)j * n + pr], pv);
-        if (lane == 0) *sh_pv = pv;
+      wkey = __reduce_max_sync(0xffffffffu, key);
+    };
+    if (active) search();
+    // The current column is always register column 0: a step writes column q to
+    // register column q - 1 and the finished column to the last one, so the loop
+    // is not unrolled.
+#pragma unroll 1
+    for (int j = 0; j < sw; ++j) {
+      const int buf = (j & 1) * NW;
+      if (lane == 0) reinterpret_cast<unsigned*>(part)[buf + warp] = wkey;
+      if (key == wkey && key != 0u) {
+        cplx* ws = slot + (buf + warp) * SW;
+#pragma unroll
+        for (int k = 0; k < RT; ++k)
+          if (RT == 1 || tid + k * T == 1023 - (int)(key & 1023u))
+#pragma unroll
+            for (int q = 1; q < SW; ++q) ws[q] = a[k][q];
+        ws[0] = gj_pivot_inv(cand);
       }
+      __syncthreads();
+      unsigned best = 0;
+#pragma unroll
+      for (int q = 0; q < NW / 4; ++q) {
+        const uint4 x = part[buf / 4 + q];
+        best = max(max(best, max(x.x, x.y)), max(x.z, x.w));
+      }
+      const int pr = 1023 - (int)(best & 1023u);
+      if (best == 0u) {  // no candidate row (uniform)
+        dead = true;
+        if (tid == 0) sh_piv[s0 + j] = -1;
+        if (tid == 0 && p.info) atomicCAS(p.info, 0, k0 + s0 + j + 1);
+        break;
+      }
+      const cplx* row = slot + (buf + ((pr % T) >> 5)) * SW;
+      if (tid == 0) {
+        sh_piv[s0 + j] = pr;
+        at[pr] = (uint8_t)(s0 / SW);
+        if (p.info && row[0].x == 0.0 && row[0].y == 0.0) atomicCAS(p.info, 0, k0 + s0 + j + 1);  // zero pivot
+      }
+      if (!active) continue;
+      // row r -= f row(pivot) with f = a[r][j] / pivot; the pivot row itself is
+      // 0 - (-1/pivot) row(pivot)
+      const cplx pv = row[0];
+      cplx f[RT];
+      bool prow[RT];
+#pragma unroll
+      for (int k = 0; k < RT; ++k) {
+        f[k] = cmul(a[k][0], pv);
+        prow[k] = tid + k * T == pr;
+        used[k] = used[k] || prow[k];
+        if (prow[k]) f[k] = cneg(pv);
+      }
+      // the next column goes first, so that its search overlaps the others' arithmetic
+#pragma unroll
+      for (int q = 1; q < SW; ++q) {
+        const cplx x = row[q];
+#pragma unroll
+        for (int k = 0; k < RT; ++k)
+          a[k][q - 1] = gj_cfms(prow[k] ? make_double2(0.0, 0.0) : a[k][q], f[k], x);
+        if (q == 1) search();
+      }
+#pragma unroll
+      for (int k = 0; k < RT; ++k) a[k][SW - 1] = cneg(f[k]);
+    }
+    // column j of the sub-panel is register column SW - sw + j
+#pragma unroll
+    for (int k = 0; k < RT; ++k)
+#pragma unroll
+      for (int q = 0; q < SW; ++q) {
+        const int r = tid + k * T, j = q - (SW - sw);
+        if (r < n && j >= 0) S[(size_t)(s0 + j) * ldw + r] = a[k][q];
+      }
+    __syncthreads();
+    if (dead || wt == 1) continue;
+    // the pivot rows in the other columns (unused k of a last, narrower tile: zero)
+    for (int i = tid; i < SW * SW * wt; i += T) {
+      const int q = i / SW, j = i % SW;
+      Bb[q * SW + (j ^ ((q & 1) << 2))] =
+          q < w && j < sw ? S[(size_t)q * ldw + sh_piv[s0 + j]] : make_double2(0.0, 0.0);
     }
     __syncthreads();
-    const int pr = sh_piv[c];
-    if (pr < 0) break;  // no candidate row: the host reports the info code
-    const cplx pv = *sh_pv;
-    for (int j = warp; j < w; j += NW) {
-      const cplx rj = rowbuf[j];
-      cplx* Sj = S + (size_t)j * n;
-      if (j == c) {
-        for (int r = lane; r < n; r += 32) Sj[r] = (r == pr) ? rj : cneg(cmul(colbuf[r], pv));
-      } else {
-        for (int r = lane; r < n; r += 32) Sj[r] = (r == pr) ? rj : cfms(Sj[r], colbuf[r], rj);
+    // rank-8 update of the other column tiles: warps take row tiles of 16 and,
+    // with fewer row tiles than warps, share the column tiles of one
+    const int mt = (n + 15) / 16, ng = mt >= NW ? 1 : NW / mt;
+    const int g = lane >> 2, tq = lane & 3, ks = s0 / SW;
+    const int m_step = mt >= NW ? NW : mt;
+    if (warp < m_step * ng)
+      for (int m = warp % m_step; m < mt; m += m_step) {
+        const int r0 = m * 16 + g, r1 = r0 + 8;
+        const bool i0 = r0 < n, i1 = r1 < n;
+        double ar[2][2], ai[2][2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int kk = tq + 4 * h;
+          cplx x0 = make_double2(0.0, 0.0), x1 = x0;
+          if (kk < sw && i0) x0 = S[(size_t)(s0 + kk) * ldw + r0];
+          if (kk < sw && i1) x1 = S[(size_t)(s0 + kk) * ldw + r1];
+          ar[h][0] = x0.x; ai[h][0] = x0.y;
+          ar[h][1] = x1.x; ai[h][1] = x1.y;
+        }
+        // the next tile's values (zero at the sub-panel's pivot rows) are read
+        // while this tile's products run
+        const bool o0 = i0 && at[r0] != ks, o1 = i1 && at[r1] != ks;
+        cplx c[4], b[2], cn[4], bn[2];
+        auto load = [&](int u, cplx (&cc)[4], cplx (&bb)[2]) {
+          const int ct = u + (u >= ks ? 1 : 0);
+          const cplx* C0 = S + (size_t)(ct * SW + 2 * tq) * ldw + r0;
+          const cplx z = make_double2(0.0, 0.0);
+          cc[0] = o0 ? C0[0] : z;
+          cc[1] = o0 ? C0[ldw] : z;
+          cc[2] = o1 ? C0[8] : z;
+          cc[3] = o1 ? C0[ldw + 8] : z;
+          const cplx* B = Bb + (size_t)(ct * SW + g) * SW;
+          bb[0] = B[tq ^ ((g & 1) << 2)];
+          bb[1] = B[(tq + 4) ^ ((g & 1) << 2)];
+        };
+        const int u0 = warp / m_step;
+        if (u0 < wt - 1) load(u0, c, b);
+        for (int u = u0; u < wt - 1; u += ng) {
+          if (u + ng < wt - 1) load(u + ng, cn, bn);
+          double re[4], im[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            re[e] = c[e].x;
+            im[e] = c[e].y;
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            gj_dmma(re, ar[h][0], ar[h][1], b[h].x);
+            gj_dmma(im, ar[h][0], ar[h][1], b[h].y);
+            gj_dmma(re, ai[h][0], ai[h][1], -b[h].y);
+            gj_dmma(im, ai[h][0], ai[h][1], b[h].x);
+          }
+          cplx* C0 = S + (size_t)((u + (u >= ks ? 1 : 0)) * SW + 2 * tq) * ldw + r0;
+          if (i0) {
+            C0[0] = make_double2(re[0], im[0]);
+            C0[ldw] = make_double2(re[1], im[1]);
+          }
+          if (i1) {
+            C0[8] = make_double2(re[2], im[2]);
+            C0[ldw + 8] = make_double2(re[3], im[3]);
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) c[e] = cn[e];
+          b[0] = bn[0];
+          b[1] = bn[1];
+        }
       }
-    }
     __syncthreads();
   }
+  __syncthreads();
 
   if (!args.blocked) {
     // whole matrix in one panel: write the un-permuted inverse directly,
     // out[r, piv[c]] = S[piv[r], c]
-    bool ok = true;
-    for (int c = 0; c < w; ++c) ok = ok && sh_piv[c] >= 0;
-    if (!ok) return;  // singular: info is set, out is left untouched
+    if (dead) return;  // singular: info is set, out is left untouched
     for (int c = warp; c < n; c += NW) {
       cplx* o = p.out + (size_t)sh_piv[c] * p.ldo;
-      const cplx* Sc = S + (size_t)c * n;
+      const cplx* Sc = S + (size_t)c * ldw;
       for (int r = lane; r < n; r += 32) o[r] = Sc[sh_piv[r]];
     }
     return;
   }
   // write back slab, pivots and used flags
   for (int j = warp; j < w; j += NW)
-    for (int r = lane; r < n; r += 32) p.W[r + (size_t)(k0 + j) * p.ld] = S[(size_t)j * n + r];
-  for (int c = tid; c < w; c += GJ_THREADS) p.piv[k0 + c] = sh_piv[c];
-  for (int r = tid; r < n; r += GJ_THREADS) p.used[r] = used[r];
+    for (int r = lane; r < n; r += 32) p.W[r + (size_t)(k0 + j) * p.ld] = S[(size_t)j * ldw + r];
+  for (int c = tid; c < w; c += T) p.piv[k0 + c] = sh_piv[c];
+#pragma unroll
+  for (int k = 0; k < RT; ++k)
+    if (tid + k * T < n) p.used[tid + k * T] = used[k] ? 1 : 0;
+  if (args.blocked == 1) return;
   // F = slab - E_P  (n x w, ld n)
   for (int j = warp; j < w; j += NW) {
     const int pj = sh_piv[j];
     for (int r = lane; r < n; r += 32) {
-      cplx v = S[(size_t)j * n + r];
+      cplx v = S[(size_t)j * ldw + r];
       if (r == pj) v.x -= 1.0;
       p.F[r + (size_t)j * n] = v;
     }
   }
-  // Bbuf = W[P, :] with panel columns zeroed  (w x n, ld w); the non-panel
-  // columns of W are not modified by this kernel, so these are old values
-  for (int j = warp; j < n; j += NW) {
-    const bool inK = (j >= k0 && j < k0 + w);
-    for (int c = lane; c < w; c += 32) {
-      cplx v = make_double2(0.0, 0.0);
-      if (!inK) v = p.W[sh_piv[c] + (size_t)j * p.ld];
-      p.Bbuf[c + (size_t)j * w] = v;
-    }
+  // Bbuf = W[P, :] with panel columns zeroed  (w x n, ld w): element e = c +
+  // j w is W[piv_c, j].  The pivot rows are scattered 16-byte elements, so they
+  // are gathered with asynchronous copies (all in flight at once) over the slab,
+  // which is written back by now, and stored from there in order.
+  __syncthreads();
+  for (int e = tid; e < w * n; e += T) {
+    const int c = e % w, j = e / w;
+    gj_cp16(S + e, p.W + max(sh_piv[c], 0) + (size_t)j * p.ld);
+  }
+  gj_cp_wait();
+  for (int e = tid; e < w * n; e += T) {
+    const int j = e / w;
+    p.Bbuf[e] = j < k0 || j >= k0 + w ? S[e] : make_double2(0.0, 0.0);
   }
 }
 
-// The same panel step with the slab in registers, for blocked panels of
-// n <= 256 RT rows and nb <= 2 CT columns (RT * CT = 16 values per thread):
-// thread t owns rows r = (t >> 1) + 256 k (k < RT) and panel columns
-// (t & 1) CT .. (t & 1) CT + CT - 1.  The threads of the half that holds the
-// pivot column rotate their register columns by one after every step, so the
-// pivot column is always register column 0 (every register index is a
-// compile-time one); register column j of half h holds panel column
-// h CT + (j + rot) mod CT.  Per column: each warp reduces the arg-max of its
-// rows, every thread merges the 16 warp results (one barrier), the two threads
-// of the pivot row publish the scaled pivot row (a second barrier), and every
-// thread updates its 16 values, taking its row's pivot column value from its
-// partner lane.  Shared memory holds only the 16 partials and the pivot row;
-// the arithmetic and the pivot rule are those of zgj_panel_kernel, so the
-// results are identical.
-template <int RT, int CT>
-__global__ void __launch_bounds__(GJ_THREADS, 1)
-    zgj_panel_reg_kernel(const ZInvProblem* __restrict__ probs, GjPanelArgs args) {
-  static_assert(GJ_THREADS == 512 && RT * CT == 16, "register panel layout");
-  // fields are read where needed (not held in registers across the column loop)
-  const ZInvProblem* __restrict__ pp = probs + blockIdx.x;
-  const int n = pp->n;
-  const int k0 = args.k0;
-  if (n <= 0 || k0 >= n) return;
-  const int w = min(args.nb, n - k0);
-  constexpr int NW = GJ_THREADS / 32;
-  __shared__ double part_v[NW];
-  __shared__ int part_r[NW];
-  __shared__ cplx rowbuf[2 * CT];
-  __shared__ cplx sh_pv;
-  __shared__ int sh_piv[2 * CT];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = tid & 1, rr = tid >> 1;
-  if (tid < 2 * CT) sh_piv[tid] = 0;  // valid row indices even if the column loop stops early
-
-  cplx a[RT][CT];
-  bool used[RT];
-  {
-    const cplx* W = pp->W;
-    const int ld = pp->ld;
-#pragma unroll
-    for (int k = 0; k < RT; ++k) {
-      const int r = rr + 256 * k;
-      used[k] = r >= n || (k0 > 0 && pp->used[r]);
-#pragma unroll
-      for (int j = 0; j < CT; ++j) {
-        const int col = h * CT + j;
-        a[k][j] = (r < n && col < w) ? W[r + (size_t)(k0 + col) * ld] : make_double2(0.0, 0.0);
-      }
+// The rank-w update after a panel, in place: W[:, j] += S W[P, j] for the columns
+// j outside the panel, without the old value at the pivot rows P; S is the
+// panel's slab W[:, k0 .. k0 + w).  A CTA owns BN columns of one matrix and all
+// of its rows: it gathers its part of the pivot rows first (nobody else writes
+// those columns), then takes row tiles of 64, with the next tile's S rows in
+// flight while it multiplies (3M products on the FP64 tensor path, as in the
+// batched GEMM).
+// Bounds: FP64 tensor time (8 n^2 w flops per matrix at 3/4) against 32 n^2
+// bytes of W from L2 or HBM.  64 matrices of 256, w = 32: 53 us, 20 TFLOP/s of
+// 8 n^2 w (69 us with the pivot rows staged through memory by the panel and
+// the batched GEMM, whose gather also cost the panel 16 us).  BN = 32 for
+// batches that fill the GPU; 16 columns when there are fewer CTAs than two per
+// SM, since a CTA's row tiles run one after the other (one matrix: 15 us).
+template <int BN>
+__global__ void __launch_bounds__(256, 2)
+    zgj_update_kernel(const ZInvProblem* __restrict__ probs, int k0, int nb, int stripes) {
+  constexpr int BM = 64, ALD = BM + 2, BLD = 36, NI = BN / 16;
+  const int prob = blockIdx.x / stripes, c0 = (blockIdx.x - prob * stripes) * BN;
+  const ZInvProblem& pp = probs[prob];
+  const int n = pp.n, ld = pp.ld;
+  if (c0 >= n || k0 >= n) return;
+  const int w = min(nb, n - k0);
+  if (c0 >= k0 && min(c0 + BN, n) <= k0 + w) return;  // the panel's own columns
+  cplx* const W = pp.W;
+  const int* const piv = pp.piv + k0;
+  const int kp = (w + 3) & ~3;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx* As = reinterpret_cast<cplx*>(smem_raw);  // [2][nb][ALD]: S rows of a tile, As[k][m]
+  cplx* Bs = As + 2 * (size_t)((nb + 3) & ~3) * ALD;  // [BN][BLD]: pivot rows, Bs[n][k]
+  uint8_t* isp = reinterpret_cast<uint8_t*>(Bs + BN * BLD);  // n: pivot rows of this panel
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
+  auto load_a = [&](int rt, int buf) {
+    cplx* A = As + (size_t)buf * ((nb + 3) & ~3) * ALD;
+    for (int i = tid; i < kp * BM; i += 256) {
+      const int r = i % BM, kk = i / BM, gr = rt * BM + r;
+      gj_cp16z(A + kk * ALD + r, W + gr + (size_t)(k0 + kk) * ld, gr < n && kk < w, W);
     }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  load_a(0, 0);
+  for (int i = tid; i < BN * kp; i += 256) {
+    const int kk = i % kp, c = i / kp;
+    const bool in = kk < w && c0 + c < n;
+    const int pr = in ? max(piv[kk], 0) : 0;
+    gj_cp16z(Bs + c * BLD + kk, W + pr + (size_t)(c0 + c) * ld, in, W);
   }
-
-  int rot = 0;  // rotations of this thread's register columns
-  for (int c = 0; c < w; ++c) {
-    const bool mine = h == (c >= CT ? 1 : 0);
-    // 1. arg-max of |re| + |im| over this thread's unused rows of column c
-    double bv = -1.0;
-    int br = -1;
-    if (mine)
-#pragma unroll
-      for (int k = 0; k < RT; ++k)
-        if (!used[k]) argmax_merge(bv, br, cabs1(a[k][0]), rr + 256 * k);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const double v2 = __shfl_xor_sync(0xffffffffu, bv, off);
-      const int r2 = __shfl_xor_sync(0xffffffffu, br, off);
-      argmax_merge(bv, br, v2, r2);
-    }
-    if (lane == 0) {
-      part_v[warp] = bv;
-      part_r[warp] = br;
-    }
-    __syncthreads();
-    // 2. every thread merges the warp results (one order for all): one pivot
-    bv = part_v[0];
-    br = part_r[0];
-#pragma unroll
-    for (int q = 1; q < NW; ++q) argmax_merge(bv, br, part_v[q], part_r[q]);
-    const int pr = br;
-    if (pr < 0 || bv == 0.0) {
-      if (tid == 0 && pp->info) atomicCAS(pp->info, 0, k0 + c + 1);
-      if (pr < 0) break;  // uniform: the host reports the info code
-    }
-    // 3. the pivot column value of each of this thread's rows (register column
-    //    0 of the partner that holds column c), then the two threads of row pr
-    //    publish the pivot inverse and the scaled pivot row
-    const int kp = pr >> 8;
-    cplx cv[RT];
-#pragma unroll
-    for (int k = 0; k < RT; ++k) {
-      cplx o;
-      o.x = __shfl_xor_sync(0xffffffffu, a[k][0].x, 1);
-      o.y = __shfl_xor_sync(0xffffffffu, a[k][0].y, 1);
-      cv[k] = mine ? a[k][0] : o;
-    }
-    if (rr == (pr & 255)) {
-      cplx pivv = cv[0];
-#pragma unroll
-      for (int k = 1; k < RT; ++k)
-        if (k == kp) pivv = cv[k];
-      const cplx pv = (pivv.x == 0.0 && pivv.y == 0.0) ? make_double2(0.0, 0.0) : cinv(pivv);
-#pragma unroll
-      for (int j = 0; j < CT; ++j) {
-        cplx sj = a[0][j];
-#pragma unroll
-        for (int k = 1; k < RT; ++k)
-          if (k == kp) sj = a[k][j];
-        const int jj = j + rot < CT ? j + rot : j + rot - CT;
-        rowbuf[h * CT + jj] = (mine && j == 0) ? pv : cmul(sj, pv);
-      }
-      if (mine) {
-        sh_pv = pv;
-        sh_piv[c] = pr;
-      }
-#pragma unroll
-      for (int k = 0; k < RT; ++k)
-        if (k == kp) used[k] = true;
-    }
-    __syncthreads();
-    // 4. the Gauss-Jordan step on this thread's values (the pivot row is read
-    //    element by element, so its values are not all held in registers)
-    const cplx pv = sh_pv;
-    const volatile double* rb = reinterpret_cast<const volatile double*>(rowbuf + h * CT);
-#pragma unroll
-    for (int k = 0; k < RT; ++k) {
-      const bool prow = rr + 256 * k == pr;
-#pragma unroll
-      for (int j = 0; j < CT; ++j) {
-        const int jj = j + rot < CT ? j + rot : j + rot - CT;
-        const cplx rj = make_double2(rb[2 * jj], rb[2 * jj + 1]);
-        if (prow) a[k][j] = rj;
-        else if (mine && j == 0) a[k][j] = cneg(cmul(cv[k], pv));
-        else a[k][j] = cfms(a[k][j], cv[k], rj);
-      }
-    }
-    // 5. the pivot half brings its next column to register column 0
-    if (mine) {
-#pragma unroll
-      for (int k = 0; k < RT; ++k) {
-        const cplx t = a[k][0];
-#pragma unroll
-        for (int j = 0; j + 1 < CT; ++j) a[k][j] = a[k][j + 1];
-        a[k][CT - 1] = t;
-      }
-      rot = rot + 1 == CT ? 0 : rot + 1;
-    }
-    // the next column's partials overwrite part_v only after every thread
-    // passed the barrier above, and rowbuf only after the next one
-  }
+  asm volatile("cp.async.commit_group;\n" ::);
+  for (int r = tid; r < n; r += 256) isp[r] = 0;
   __syncthreads();
-  // write back slab, pivots, used flags and F = slab - E_P (n x w, ld n)
-  {
-    cplx* W = pp->W;
-    cplx* F = pp->F;
-    const int ld = pp->ld;
+  if (tid < w && piv[tid] >= 0) isp[piv[tid]] = 1;
+  const int wm = (warp & 3) * 16, wn = (warp >> 2) * (BN / 2);
+  const int nrt = (n + BM - 1) / BM;
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  for (int rt = 0; rt < nrt; ++rt) {
+    if (rt + 1 < nrt) load_a(rt + 1, (rt + 1) & 1);
+    // the old values of this warp's 16 x BN/2 part (zero at pivot rows)
+    cplx old[NI][4];
 #pragma unroll
-    for (int k = 0; k < RT; ++k) {
-      const int r = rr + 256 * k;
-      if (r >= n) continue;
+    for (int x = 0; x < NI; ++x)
 #pragma unroll
-      for (int j = 0; j < CT; ++j) {
-        const int jj = j + rot < CT ? j + rot : j + rot - CT;
-        const int col = h * CT + jj;
-        if (col >= w) continue;
-        cplx v = a[k][j];
-        W[r + (size_t)(k0 + col) * ld] = v;
-        if (r == sh_piv[col]) v.x -= 1.0;
-        F[r + (size_t)col * n] = v;
+      for (int e = 0; e < 4; ++e) {
+        const int r = rt * BM + wm + g + ((e >> 1) << 3), c = c0 + wn + x * 8 + 2 * tq + (e & 1);
+        old[x][e] = r < n && c < n && !isp[r] ? W[r + (size_t)c * ld] : make_double2(0.0, 0.0);
       }
-      if (h == 0) pp->used[r] = used[k] ? 1 : 0;
-    }
-  }
-  for (int c = tid; c < w; c += GJ_THREADS) pp->piv[k0 + c] = sh_piv[c];
-  // Bbuf = W[P, :] with panel columns zeroed  (w x n, ld w): element e = c +
-  // j w is W[piv_c, j]; the pivot rows are scattered, so every thread keeps
-  // GU gathers in flight before it stores them
-  {
-    const cplx* W = pp->W;
-    cplx* Bbuf = pp->Bbuf;
-    const int ld = pp->ld;
-    const int total = w * n;
-    constexpr int GU = 8;
-    for (int e0 = tid; e0 < total; e0 += GU * GJ_THREADS) {
-      cplx v[GU];
+    double P1[NI][4] = {}, P2[NI][4] = {}, P3[NI][4] = {};
+    const cplx* A = As + (size_t)(rt & 1) * ((nb + 3) & ~3) * ALD + wm + g;
+    const cplx* B = Bs + (wn + g) * BLD + tq;
+#pragma unroll 2
+    for (int kk = 0; kk < kp; kk += 4) {
+      const cplx x0 = A[(kk + tq) * ALD], x1 = A[(kk + tq) * ALD + 8];
+      const double s0 = x0.x + x0.y, s1 = x1.x + x1.y;
 #pragma unroll
-      for (int u = 0; u < GU; ++u) {
-        const int e = e0 + u * GJ_THREADS;
-        v[u] = make_double2(0.0, 0.0);
-        if (e < total) {
-          const int c = e % w, j = e / w;
-          if (j < k0 || j >= k0 + w) v[u] = W[sh_piv[c] + (size_t)j * ld];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < GU; ++u) {
-        const int e = e0 + u * GJ_THREADS;
-        if (e < total) Bbuf[e] = v[u];
+      for (int x = 0; x < NI; ++x) {
+        const cplx y = B[x * 8 * BLD + kk];
+        gj_dmma(P1[x], x0.x, x1.x, y.x);
+        gj_dmma(P2[x], x0.y, x1.y, y.y);
+        gj_dmma(P3[x], s0, s1, y.x + y.y);
       }
     }
+#pragma unroll
+    for (int x = 0; x < NI; ++x)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int r = rt * BM + wm + g + ((e >> 1) << 3), c = c0 + wn + x * 8 + 2 * tq + (e & 1);
+        if (r < n && c < n && (c < k0 || c >= k0 + w))
+          W[r + (size_t)c * ld] = make_double2(old[x][e].x + (P1[x][e] - P2[x][e]),
+                                               old[x][e].y + (P3[x][e] - P1[x][e] - P2[x][e]));
+      }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
   }
 }
 
@@ -363,28 +469,44 @@ __global__ void zgj_unpermute_kernel(const ZInvProblem* __restrict__ probs) {
 }
 
 size_t zgj_panel_smem_bytes(int n, int nb) {
-  int w = nb < n ? nb : n;
-  size_t b = (size_t)n * w * sizeof(cplx) + (size_t)n * sizeof(cplx) + (size_t)w * sizeof(cplx);
-  b += (GJ_THREADS / 32) * (sizeof(double) + sizeof(int)) + (size_t)w * sizeof(int) + (size_t)n;
+  const size_t w = nb < n ? nb : n, w8 = (w + gj::SW - 1) / gj::SW * gj::SW;
+  size_t b = (size_t)(n | 1) * w8 * sizeof(cplx) + w8 * gj::SW * sizeof(cplx);
+  b += 2 * 8 * (gj::SW * sizeof(cplx) + sizeof(unsigned)) + w * sizeof(int) + n;
   return (b + 15) & ~size_t(15);
 }
 
+// One thread per row up to 256 rows, then two and four rows per thread.  Up to
+// 128 rows four warps, whose barriers are cheaper and whose CTAs share an SM --
+// except a whole matrix above 64, whose rank-8 updates want eight warps (n =
+// 100: 131 us against 162 us; n = 64: 64 us both, 592 matrices 152 against 137).
 cudaError_t launch_zgj_panel(const ZInvProblem* probs_dev, int nprob, int k0, int nb, int blocked, size_t smem,
                              cudaStream_t stream, int max_n) {
   if (nprob <= 0) return cudaSuccess;
   GjPanelArgs a{k0, nb, blocked};
-  // blocked panels of up to 256 rows x 32 columns or 512 rows x 16 columns:
-  // the slab in registers
-  if (blocked && max_n > 0 && max_n <= 256 && nb <= 32)
-    zgj_panel_reg_kernel<1, 16><<<nprob, GJ_THREADS, 0, stream>>>(probs_dev, a);
-  else if (blocked && max_n > 0 && max_n <= 512 && nb <= 16)
-    zgj_panel_reg_kernel<2, 8><<<nprob, GJ_THREADS, 0, stream>>>(probs_dev, a);
-  else
-    zgj_panel_kernel<<<nprob, GJ_THREADS, smem, stream>>>(probs_dev, a);
+  if (max_n <= (blocked ? 128 : 64)) zgj_panel_kernel<128, 1><<<nprob, 128, smem, stream>>>(probs_dev, a);
+  else if (max_n <= 256) zgj_panel_kernel<256, 1><<<nprob, 256, smem, stream>>>(probs_dev, a);
+  else if (max_n <= 512) zgj_panel_kernel<256, 2><<<nprob, 256, smem, stream>>>(probs_dev, a);
+  else zgj_panel_kernel<256, 4><<<nprob, 256, smem, stream>>>(probs_dev, a);
   return cudaGetLastError();
 }
 
-// Raise the dynamic shared-memory limit of the panel kernel (outside capture).
+static size_t zgj_update_smem_bytes(int max_n, int nb, int bn) {
+  return (2 * (size_t)((nb + 3) & ~3) * 66 + (size_t)bn * 36) * sizeof(cplx) + ((max_n + 15) & ~15);
+}
+
+cudaError_t launch_zgj_update(const ZInvProblem* probs_dev, int nprob, int k0, int nb, int max_n, cudaStream_t stream) {
+  if (nprob <= 0) return cudaSuccess;
+  const int s32 = (max_n + 31) / 32;
+  if ((long long)nprob * s32 >= 2 * 148) {
+    zgj_update_kernel<32><<<nprob * s32, 256, zgj_update_smem_bytes(max_n, nb, 32), stream>>>(probs_dev, k0, nb, s32);
+  } else {
+    const int s16 = (max_n + 15) / 16;
+    zgj_update_kernel<16><<<nprob * s16, 256, zgj_update_smem_bytes(max_n, nb, 16), stream>>>(probs_dev, k0, nb, s16);
+  }
+  return cudaGetLastError();
+}
+
+// Raise the dynamic shared-memory limit of the panel kernels (outside capture).
 // The attribute is process-wide, so it is always set to the device's opt-in
 // maximum: a later, smaller request never lowers the limit another live plan
 // relies on.
@@ -394,7 +516,11 @@ cudaError_t zgj_prepare(size_t smem) {
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&mx, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
   if (smem > (size_t)mx) return cudaErrorInvalidValue;
-  return cudaFuncSetAttribute(zgj_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+  for (const void* f : {(const void*)zgj_panel_kernel<128, 1>, (const void*)zgj_panel_kernel<256, 1>,
+                        (const void*)zgj_panel_kernel<256, 2>, (const void*)zgj_panel_kernel<256, 4>,
+                        (const void*)zgj_update_kernel<16>, (const void*)zgj_update_kernel<32>})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+  return e;
 }
 
 cudaError_t launch_zgj_unpermute(const ZInvProblem* probs_dev, int nprob, int max_n, cudaStream_t stream) {

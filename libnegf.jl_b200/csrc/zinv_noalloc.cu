@@ -171,12 +171,12 @@ extern "C" int negf_zinv_batched_noalloc(int32_t nprob, const int32_t* n, void* 
   if (e != cudaSuccess) return cuda_fail(e, "negf_zinv_batched_noalloc: copy");
   const ZInvProblem* dinv = reinterpret_cast<const ZInvProblem*>(at(o_inv));
   if (!blocked) {
-    e = launch_zgj_panel(dinv, cnt, 0, nb, 0, zgj_panel_smem_bytes(max_n, nb), st);
+    e = launch_zgj_panel(dinv, cnt, 0, nb, 0, zgj_panel_smem_bytes(max_n, nb), st, max_n);
     if (e != cudaSuccess) return cuda_fail(e, "negf_zinv_batched_noalloc: panel");
   } else {
     for (int p = 0; p < npanels; ++p) {
       const int k0 = p * nb;
-      e = launch_zgj_panel(dinv, cnt, k0, nb, 1, zgj_panel_smem_bytes(max_n, nb), st);
+      e = launch_zgj_panel(dinv, cnt, k0, nb, 2, zgj_panel_smem_bytes(max_n, nb), st, max_n);
       if (e != cudaSuccess) return cuda_fail(e, "negf_zinv_batched_noalloc: panel");
       std::vector<ZGemmProblem> g;
       std::vector<int> ts;
