@@ -20,7 +20,7 @@ inline ZGemmProblem gp(const cplx* A, int lda, const cplx* B, int ldb, cplx* C, 
                        cplx alpha, const cplx* Cin = nullptr, int ldcin = 1, cplx beta = {0.0, 0.0},
                        cplx diag = {0.0, 0.0}) {
   ZGemmProblem p;
-  p.A = A; p.B = B; p.Cin = Cin; p.C = C; p.diag_ptr = nullptr;
+  p.A = A; p.B = B; p.Cin = Cin; p.C = C; p.diag_ptr = nullptr; p.alpha_ptr = nullptr;
   p.m = m; p.n = n; p.k = k;
   p.lda = lda > 0 ? lda : 1; p.ldb = ldb > 0 ? ldb : 1; p.ldc = ldc; p.ldcin = ldcin > 0 ? ldcin : 1;
   p.pad_ = 0;
@@ -387,7 +387,7 @@ void Plan::gemm_mixed(char opA, char opB, const std::vector<ZGemmProblem>& probs
     const int a = which[i].first, b = which[i].second;
     OzMmaProblem q;
     q.SA = slc[a]; q.eA = exs[a]; q.SB = slc[b]; q.eB = exs[b];
-    q.C = p.C; q.Cin = p.Cin; q.diag_ptr = p.diag_ptr;
+    q.C = p.C; q.Cin = p.Cin; q.diag_ptr = p.diag_ptr; q.alpha_ptr = p.alpha_ptr;
     q.m = p.m; q.n = p.n; q.m_pad = rpad[a]; q.n_pad = rpad[b]; q.k_pad = kpad[a];
     q.ldc = p.ldc; q.ldcin = p.ldcin; q.pad_ = 0;
     q.alpha = p.alpha; q.beta = p.beta; q.diag = p.diag;
@@ -834,7 +834,7 @@ static InvSpec inv_spec(const TriSystem& s, RgfWork& w, int i) {
   return sp;
 }
 
-void build_rgf_upward(Plan& plan, const std::vector<TriSystem>& sys, std::vector<RgfWork>& work) {
+void build_rgf_upward(Plan& plan, const std::vector<TriSystem>& sys, std::vector<RgfWork>& work, GnUpward* gn) {
   int maxN = 0;
   for (const auto& s : sys) maxN = std::max(maxN, s.npl());
   // bottom layer: X_{N-1} = M[N-1,N-1]  (rgf.jl:144)
@@ -853,12 +853,14 @@ void build_rgf_upward(Plan& plan, const std::vector<TriSystem>& sys, std::vector
     plan.gemm('N', 'N', pr);
     plan.inv(iv);
   }
-  for (int j = 1; j < maxN; ++j) {
+  // the last round only finishes the operator of the topmost layers (gn)
+  for (int j = 1; j < maxN + (gn ? 1 : 0); ++j) {
     // R_i = M[i,i+1] g_{i+1}  (rgf.jl:152-154) and L_{i+1} = g_{i+1} M[i+1,i]  (rgf.jl:157)
     std::vector<ZGemmProblem> rN, lN, lC;
     for (size_t k = 0; k < sys.size(); ++k) {
       const auto& s = sys[k];
       int i = s.npl() - 1 - j;
+      if (gn && i >= -1) gn->after(s, work[k], k, i + 1, lC);
       if (i < 0) continue;
       RgfWork& w = work[k];
       rN.push_back(gp(s.U[i], s.ldU[i], w.g[i + 1], s.b[i + 1], w.R[i], s.b[i], s.b[i], s.b[i + 1], s.b[i + 1],
@@ -870,6 +872,11 @@ void build_rgf_upward(Plan& plan, const std::vector<TriSystem>& sys, std::vector
     std::vector<ZGemmProblem> nn = rN;
     nn.insert(nn.end(), lN.begin(), lN.end());
     plan.gemm('N', 'N', nn);
+    if (gn)
+      for (size_t k = 0; k < sys.size(); ++k) {
+        int i = sys[k].npl() - 1 - j;
+        if (i >= 0) gn->before(sys[k], work[k], k, i, lC);
+      }
     plan.gemm('N', 'C', lC);
     // X_i = M[i,i] - M[i,i+1] L_{i+1}  (rgf.jl:159-160), then its inverse (rgf.jl:161)
     std::vector<ZGemmProblem> xp;
@@ -882,6 +889,7 @@ void build_rgf_upward(Plan& plan, const std::vector<TriSystem>& sys, std::vector
       xp.push_back(gp(s.U[i], s.ldU[i], w.L[i], s.b[i + 1], w.W, s.b[i], s.b[i], s.b[i], s.b[i + 1],
                       cscale(s.uscale, -1.0), s.D[i], s.ldD[i], s.dscale, s.shift));
       xp.back().diag_ptr = s.shift_ptr;
+      if (gn) gn->off(s, w, k, i, xp);
       iv.push_back(inv_spec(s, w, i));
     }
     plan.gemm('N', 'N', xp);
@@ -917,8 +925,9 @@ void build_rgf_downward(Plan& plan, const std::vector<TriSystem>& sys, std::vect
       TriOut& o = out[k];
       pr.push_back(gp(o.d[i - 1], o.ldd[i - 1], w.R[i - 1], s.b[i - 1], o.u[i - 1], o.ldu[i - 1], s.b[i - 1], s.b[i],
                       s.b[i - 1], MONE));
-      pr.push_back(gp(w.L[i - 1], s.b[i], o.d[i - 1], o.ldd[i - 1], o.l[i - 1], o.ldl[i - 1], s.b[i], s.b[i - 1],
-                      s.b[i - 1], MONE));
+      if (o.l[i - 1])
+        pr.push_back(gp(w.L[i - 1], s.b[i], o.d[i - 1], o.ldd[i - 1], o.l[i - 1], o.ldl[i - 1], s.b[i], s.b[i - 1],
+                        s.b[i - 1], MONE));
     }
     plan.gemm('N', 'N', pr);
     // G[i,i] = X_i^{-1} - L_i G[i-1,i]  (rgf.jl:180-181)
@@ -966,150 +975,279 @@ void build_rgf_full_inverse(Plan& plan, const std::vector<TriSystem>& sys, std::
 // RKD (recursive Keldysh), src/keldyshndiag.jl:221-317, with every
 // be_mldivide!('N', ., ., LU(X_i)) applied as a product with g_i = X_i^{-1}.
 
+namespace {
+// Upward pass of a general Hermitian S (diagonal and upper blocks, in place,
+// keldyshndiag.jl:230-234), merged into the launches of the RGF upward pass:
+//   S[i,i] -= R_i S[i,i+1]^H;  S[i,i+1] -= R_i S[i+1,i+1];  S[i,i] -= S[i,i+1] R_i^H
+struct RkdUpward : GnUpward {
+  std::vector<HermBlocks>& S;
+  explicit RkdUpward(std::vector<HermBlocks>& s) : S(s) {}
+  void before(const TriSystem& s, RgfWork& w, size_t k, int i, std::vector<ZGemmProblem>& nc) override {
+    HermBlocks& h = S[k];
+    nc.push_back(gp(w.R[i], s.b[i], h.u[i], h.ldu[i], h.d[i], h.ldd[i], s.b[i], s.b[i], s.b[i + 1], MONE, h.d[i],
+                    h.ldd[i], ONE));
+  }
+  void off(const TriSystem& s, RgfWork& w, size_t k, int i, std::vector<ZGemmProblem>& nn) override {
+    HermBlocks& h = S[k];
+    nn.push_back(gp(w.R[i], s.b[i], h.d[i + 1], h.ldd[i + 1], h.u[i], h.ldu[i], s.b[i], s.b[i + 1], s.b[i + 1], MONE,
+                    h.u[i], h.ldu[i], ONE));
+  }
+  void after(const TriSystem& s, RgfWork& w, size_t k, int i, std::vector<ZGemmProblem>& nc) override {
+    if (i + 1 >= s.npl()) return;
+    HermBlocks& h = S[k];
+    nc.push_back(gp(h.u[i], h.ldu[i], w.R[i], s.b[i], h.d[i], h.ldd[i], s.b[i], s.b[i], s.b[i + 1], MONE, h.d[i],
+                    h.ldd[i], ONE));
+  }
+};
+
+// Upward pass of the lead operator S = Gamma_R on the last layer alone: with no
+// off-diagonal blocks the recursion is S_i = R_i S_{i+1} R_i^H, two products.
+struct LeadUpward : GnUpward {
+  std::vector<LeadSystem>& Q;
+  explicit LeadUpward(std::vector<LeadSystem>& q) : Q(q) {}
+  const cplx* op(size_t k, int i) { return i + 1 == (int)Q[k].gl.size() ? Q[k].gamR : Q[k].gl[i]; }
+  void off(const TriSystem& s, RgfWork& w, size_t k, int i, std::vector<ZGemmProblem>& nn) override {
+    nn.push_back(gp(w.R[i], s.b[i], op(k, i + 1), s.b[i + 1], Q[k].v, s.b[i], s.b[i], s.b[i + 1], s.b[i + 1], ONE));
+  }
+  void after(const TriSystem& s, RgfWork& w, size_t k, int i, std::vector<ZGemmProblem>& nc) override {
+    if (i + 1 >= s.npl()) return;
+    nc.push_back(gp(Q[k].v, s.b[i], w.R[i], s.b[i], Q[k].gl[i], s.b[i], s.b[i], s.b[i], s.b[i + 1], ONE));
+  }
+};
+}  // namespace
+
 void build_rkd(Plan& plan, const std::vector<TriSystem>& sys, std::vector<RgfWork>& work,
-               std::vector<HermBlocks>& S, const std::function<void(int)>& on_final) {
+               std::vector<HermBlocks>& S) {
   int maxN = 0;
   for (const auto& s : sys) maxN = std::max(maxN, s.npl());
-  // workspace: xb diagonal chain (npl blocks), m2/t temporaries (npl blocks each)
-  std::vector<std::vector<cplx*>> xb(sys.size()), t1(sys.size()), t2(sys.size());
+  RkdUpward up(S);
+  build_rgf_upward(plan, sys, work, &up);
+  // workspace: G_ii of M^{-1} (y), one off-diagonal block, and a temporary per layer
+  std::vector<std::vector<cplx*>> y(sys.size()), t(sys.size());
+  std::vector<cplx*> yo(sys.size());
   for (size_t k = 0; k < sys.size(); ++k) {
     const auto& s = sys[k];
-    int n = s.npl();
-    size_t tot = 0;
-    for (int i = 0; i < n; ++i) tot += 3 * (size_t)s.maxb() * s.maxb();
-    cplx* a = plan.alloc_c(tot);
-    size_t o = 0;
-    size_t bb = (size_t)s.maxb() * s.maxb();
-    for (int i = 0; i < n; ++i) {
-      xb[k].push_back(a + o); o += bb;
-      t1[k].push_back(a + o); o += bb;
-      t2[k].push_back(a + o); o += bb;
+    const size_t bb = (size_t)s.maxb() * s.maxb();
+    cplx* a = plan.alloc_c((2 * (size_t)s.npl() + 1) * bb);
+    for (int i = 0; i < s.npl(); ++i) {
+      y[k].push_back(i == 0 ? work[k].g[0] : a + 2 * i * bb);
+      t[k].push_back(a + (2 * i + 1) * bb);
     }
+    yo[k] = a + 2 * (size_t)s.npl() * bb;
   }
-  // upward RKD pass (keldyshndiag.jl:230-234), ix = N-2 .. 0
-  for (int j = 1; j < maxN; ++j) {
-    std::vector<ZGemmProblem> p1, p2, p3;
-    for (size_t k = 0; k < sys.size(); ++k) {
-      const auto& s = sys[k];
-      int i = s.npl() - 1 - j;
-      if (i < 0) continue;
-      RgfWork& w = work[k];
-      HermBlocks& h = S[k];
-      // S[i,i] -= R_i S[i,i+1]^H
-      p1.push_back(gp(w.R[i], s.b[i], h.u[i], h.ldu[i], h.d[i], h.ldd[i], s.b[i], s.b[i], s.b[i + 1], MONE, h.d[i],
-                      h.ldd[i], ONE));
-      // S[i,i+1] -= R_i S[i+1,i+1]
-      p2.push_back(gp(w.R[i], s.b[i], h.d[i + 1], h.ldd[i + 1], h.u[i], h.ldu[i], s.b[i], s.b[i + 1], s.b[i + 1],
-                      MONE, h.u[i], h.ldu[i], ONE));
-      // S[i,i] -= S[i,i+1] R_i^H
-      p3.push_back(gp(h.u[i], h.ldu[i], w.R[i], s.b[i], h.d[i], h.ldd[i], s.b[i], s.b[i], s.b[i + 1], MONE, h.d[i],
-                      h.ldd[i], ONE));
-    }
-    plan.gemm('N', 'C', p1);
-    plan.gemm('N', 'N', p2);
-    plan.gemm('N', 'C', p3);
-  }
-  // central pass, phase A: the X chain (keldyshndiag.jl:270-283)
-  //   xb[0] = I;  xb[i] = I + M[i,i-1] g_{i-1} xb[i-1] R_{i-1}
-  {
-    std::vector<ZBlockOp> ops;
-    for (size_t k = 0; k < sys.size(); ++k) {
-      const auto& s = sys[k];
-      if (s.npl() < 2) continue;
-      ZBlockOp o{};
-      o.C = xb[k][0]; o.ldc = s.b[0]; o.m = o.n = s.b[0]; o.kind = ZOP_IDENTITY; o.alpha = ONE;
-      ops.push_back(o);
-    }
-    plan.blockops(ops);
-  }
+  // central pass (keldyshndiag.jl:257-291): its chain X_i = I + M[i,i-1] g_{i-1}
+  // X_{i-1} R_{i-1}, multiplied by g_i, is the diagonal of the inverse itself,
+  // g_i X_i = g_i + L_i (g_{i-1} X_{i-1}) R_{i-1} = G_ii: two products per layer
   for (int i = 1; i + 1 < maxN; ++i) {
-    std::vector<ZGemmProblem> a1, a2, a3N, a3C;
+    std::vector<ZGemmProblem> a1, a2;
     for (size_t k = 0; k < sys.size(); ++k) {
       const auto& s = sys[k];
       if (i + 1 >= s.npl()) continue;
       RgfWork& w = work[k];
-      // m2[i-1,i] = xb[i-1] R_{i-1}  (:273)
-      a1.push_back(gp(xb[k][i - 1], s.b[i - 1], w.R[i - 1], s.b[i - 1], t1[k][i], s.b[i - 1], s.b[i - 1], s.b[i],
+      a1.push_back(gp(y[k][i - 1], s.b[i - 1], w.R[i - 1], s.b[i - 1], yo[k], s.b[i - 1], s.b[i - 1], s.b[i],
                       s.b[i - 1], ONE));
-      // xbo[i-1,i] = g_{i-1} m2[i-1,i]  (:274)
-      a2.push_back(gp(w.g[i - 1], s.b[i - 1], t1[k][i], s.b[i - 1], t2[k][i], s.b[i - 1], s.b[i - 1], s.b[i],
-                      s.b[i - 1], ONE));
-      // xb[i] = M[i,i-1] xbo[i-1,i] + I  (:275, :280-283)
-      auto p = gp(s.Lw[i - 1], s.ldL[i - 1], t2[k][i], s.b[i - 1], xb[k][i], s.b[i], s.b[i], s.b[i], s.b[i - 1],
-                  s.lscale, nullptr, 1, ZERO, ONE);
-      (s.lop == 'N' ? a3N : a3C).push_back(p);
+      a2.push_back(gp(w.L[i - 1], s.b[i], yo[k], s.b[i - 1], y[k][i], s.b[i], s.b[i], s.b[i], s.b[i - 1], ONE,
+                      w.g[i], s.b[i], ONE));
     }
     plan.gemm('N', 'N', a1);
     plan.gemm('N', 'N', a2);
-    plan.gemm('N', 'N', a3N);
-    plan.gemm('C', 'N', a3C);
   }
-  // central pass, phase B (all layers at once), keldyshndiag.jl:257-260 and :285-291:
-  //   m2[i,i] = g_i xb[i];  m2[i,i+1] = m2[i,i] S[i,i+1];  S[i,i+1] = m2[i,i+1] g_{i+1}^H
+  // S[i,i+1] = G_ii S[i,i+1] g_{i+1}^H (:285-291) and the diagonal rescale
+  // S[i,i] = g_i S[i,i] g_i^H (:296-301), all layers at once
   {
-    std::vector<ZGemmProblem> b1, b2, b3;
+    std::vector<ZGemmProblem> p1, p2;
+    std::vector<std::vector<cplx*>> t2(sys.size());
     for (size_t k = 0; k < sys.size(); ++k) {
       const auto& s = sys[k];
-      RgfWork& w = work[k];
-      HermBlocks& h = S[k];
-      for (int i = 0; i + 1 < s.npl(); ++i) {
-        b1.push_back(gp(w.g[i], s.b[i], xb[k][i], s.b[i], t1[k][i], s.b[i], s.b[i], s.b[i], s.b[i], ONE));
-        b2.push_back(gp(t1[k][i], s.b[i], h.u[i], h.ldu[i], t2[k][i], s.b[i], s.b[i], s.b[i + 1], s.b[i], ONE));
-        b3.push_back(gp(t2[k][i], s.b[i], w.g[i + 1], s.b[i + 1], h.u[i], h.ldu[i], s.b[i], s.b[i + 1], s.b[i + 1],
-                        ONE));
-      }
+      const size_t bb = (size_t)s.maxb() * s.maxb();
+      cplx* a = s.npl() > 1 ? plan.alloc_c((size_t)(s.npl() - 1) * bb) : nullptr;
+      for (int i = 0; i + 1 < s.npl(); ++i) t2[k].push_back(a + i * bb);
     }
-    plan.gemm('N', 'N', b1);
-    plan.gemm('N', 'N', b2);
-    plan.gemm('N', 'C', b3);
-  }
-  // diagonal rescale (keldyshndiag.jl:296-301): S[i,i] = g_i S[i,i] g_i^H
-  {
-    std::vector<ZGemmProblem> c1, c2;
     for (size_t k = 0; k < sys.size(); ++k) {
       const auto& s = sys[k];
       RgfWork& w = work[k];
       HermBlocks& h = S[k];
       for (int i = 0; i < s.npl(); ++i) {
-        c1.push_back(gp(w.g[i], s.b[i], h.d[i], h.ldd[i], t1[k][i], s.b[i], s.b[i], s.b[i], s.b[i], ONE));
-        c2.push_back(gp(t1[k][i], s.b[i], w.g[i], s.b[i], h.d[i], h.ldd[i], s.b[i], s.b[i], s.b[i], ONE));
+        p1.push_back(gp(w.g[i], s.b[i], h.d[i], h.ldd[i], t[k][i], s.b[i], s.b[i], s.b[i], s.b[i], ONE));
+        p2.push_back(gp(t[k][i], s.b[i], w.g[i], s.b[i], h.d[i], h.ldd[i], s.b[i], s.b[i], s.b[i], ONE));
+        if (i + 1 == s.npl()) continue;
+        p1.push_back(gp(y[k][i], s.b[i], h.u[i], h.ldu[i], t2[k][i], s.b[i], s.b[i], s.b[i + 1], s.b[i], ONE));
+        p2.push_back(gp(t2[k][i], s.b[i], w.g[i + 1], s.b[i + 1], h.u[i], h.ldu[i], s.b[i], s.b[i + 1], s.b[i + 1],
+                        ONE));
       }
     }
-    plan.gemm('N', 'N', c1);
-    plan.gemm('N', 'C', c2);
+    plan.gemm('N', 'N', p1);
+    plan.gemm('N', 'C', p2);
   }
-  // downward RKD pass (keldyshndiag.jl:313-317), ix = 0 .. N-2
-  for (int i = 0; i + 1 < maxN; ++i) {
-    std::vector<ZGemmProblem> d1, d2, d3;
+  // downward RKD pass (keldyshndiag.jl:313-317), ix = 0 .. N-2:
+  //   S[i+1,i+1] -= S[i,i+1]^H L_{i+1}^H, for all layers at once (it takes
+  //   S[i,i+1] as the central pass left it), then layer by layer
+  //   S[i,i+1] -= S[i,i] L_{i+1}^H;  S[i+1,i+1] -= L_{i+1} S[i,i+1]
+  {
+    std::vector<ZGemmProblem> d1;
     for (size_t k = 0; k < sys.size(); ++k) {
       const auto& s = sys[k];
-      if (i + 1 >= s.npl()) continue;
       RgfWork& w = work[k];
       HermBlocks& h = S[k];
-      // S[i+1,i+1] -= S[i,i+1]^H L_{i+1}^H
-      d1.push_back(gp(h.u[i], h.ldu[i], w.L[i], s.b[i + 1], h.d[i + 1], h.ldd[i + 1], s.b[i + 1], s.b[i + 1], s.b[i],
-                      MONE, h.d[i + 1], h.ldd[i + 1], ONE));
-      // S[i,i+1] -= S[i,i] L_{i+1}^H
-      d2.push_back(gp(h.d[i], h.ldd[i], w.L[i], s.b[i + 1], h.u[i], h.ldu[i], s.b[i], s.b[i + 1], s.b[i], MONE,
-                      h.u[i], h.ldu[i], ONE));
+      for (int i = 0; i + 1 < s.npl(); ++i)
+        d1.push_back(gp(h.u[i], h.ldu[i], w.L[i], s.b[i + 1], h.d[i + 1], h.ldd[i + 1], s.b[i + 1], s.b[i + 1], s.b[i],
+                        MONE, h.d[i + 1], h.ldd[i + 1], ONE));
     }
     plan.gemm('C', 'C', d1);
-    plan.gemm('N', 'C', d2);
-    std::vector<ZGemmProblem> d3v;
+  }
+  for (int i = 0; i + 1 < maxN; ++i) {
+    std::vector<ZGemmProblem> d2, d3;
     for (size_t k = 0; k < sys.size(); ++k) {
       const auto& s = sys[k];
       if (i + 1 >= s.npl()) continue;
       RgfWork& w = work[k];
       HermBlocks& h = S[k];
-      // S[i+1,i+1] -= L_{i+1} S[i,i+1]
-      d3v.push_back(gp(w.L[i], s.b[i + 1], h.u[i], h.ldu[i], h.d[i + 1], h.ldd[i + 1], s.b[i + 1], s.b[i + 1], s.b[i],
-                       MONE, h.d[i + 1], h.ldd[i + 1], ONE));
+      d2.push_back(gp(h.d[i], h.ldd[i], w.L[i], s.b[i + 1], h.u[i], h.ldu[i], s.b[i], s.b[i + 1], s.b[i], MONE,
+                      h.u[i], h.ldu[i], ONE));
+      d3.push_back(gp(w.L[i], s.b[i + 1], h.u[i], h.ldu[i], h.d[i + 1], h.ldd[i + 1], s.b[i + 1], s.b[i + 1], s.b[i],
+                      MONE, h.d[i + 1], h.ldd[i + 1], ONE));
     }
-    plan.gemm('N', 'N', d3v);
-    // iteration i last reads S[i,i] (d2)
-    if (on_final) on_final(i);
+    plan.gemm('N', 'C', d2);
+    plan.gemm('N', 'N', d3);
   }
-  if (on_final && maxN > 0) on_final(maxN - 1);
+}
+
+// ---------------------------------------------------------------------------
+// G^R and G^< diagonals and the transmission of lead-driven systems.
+//
+// Sigma^in = f_L Gamma_L on layer 0 and f_R Gamma_R on layer N-1, so the
+// Hermitian operator of keldyshndiag! has no off-diagonal blocks and stays a
+// chain (S_i = R_i .. R_{N-2} Gamma_R (..)^H); its products share work with
+// those of G^R.  Per layer 13 products of 8 b^3 flops (21 in the general
+// sequence with the blocks of G^R below the diagonal: 32 x 256, 64 energies,
+// FP64 194 -> 134 ms, mixed 131 -> 87 ms), in 4 + 4 launches:
+//   up (with the RGF pass): v = R_i S_{i+1};  S_i = v R_i^H
+//   all layers:             t_i = f_R S_i g_i^H (i = 0: + f_L Gamma_L g_0^H);  n_i = g_i t_i
+//   down:                   G_{i,i+1} = -G_ii R_i;  G_{i+1,i+1} = g_{i+1} - L_{i+1} G_{i,i+1}
+//                           A = G_{i,i+1} t_{i+1} - G^n_ii L_{i+1}^H / 2
+//                           G^n_{i+1,i+1} = n_{i+1} - L_{i+1} A - (L_{i+1} A)^H
+// (the last two are keldyshndiag.jl:313-317 with both updates of S[i+1,i+1] as
+// one product and its conjugate transpose), and beside them G_{0,i+1} =
+// -G_{0,i} R_i for T = Re Tr[Gamma_L G_{0,N-1} Gamma_R G_{0,N-1}^H] (from S_0,
+// T would need no chain, but its error doubled).
+void build_lead_pass(Plan& plan, const std::vector<TriSystem>& sys, std::vector<RgfWork>& work,
+                     std::vector<LeadSystem>& Q, const std::function<void(int)>& gr_final,
+                     const std::function<void(int)>& gl_final) {
+  int maxN = 0;
+  const size_t ns = sys.size();
+  for (const auto& s : sys) maxN = std::max(maxN, s.npl());
+  std::vector<std::vector<cplx*>> t(ns);
+  std::vector<cplx*> u(ns), ub(ns), q(ns);
+  std::vector<std::vector<cplx*>> y(ns);  // G_{0,i} (two in turn), and the two factors of the trace
+  std::vector<std::vector<cplx*>> G(ns);
+  for (size_t k = 0; k < ns; ++k) {
+    const auto& s = sys[k];
+    const size_t bb = (size_t)s.maxb() * s.maxb();
+    Q[k].v = plan.alloc_c(bb);
+    u[k] = plan.alloc_c(bb);
+    ub[k] = plan.alloc_c(bb);
+    q[k] = plan.alloc_c((size_t)s.b[0] * s.b[0]);
+    if (Q[k].t_out)
+      for (int c = 0; c < 4; ++c) y[k].push_back(plan.alloc_c((size_t)s.b[0] * s.maxb()));
+    cplx* ring = Q[k].gr.empty() ? plan.alloc_c(2 * bb) : nullptr;
+    for (int i = 0; i < s.npl(); ++i) {
+      t[k].push_back(plan.alloc_c((size_t)s.b[i] * s.b[i]));
+      G[k].push_back(ring ? ring + (i & 1) * bb : Q[k].gr[i]);
+    }
+  }
+  LeadUpward up(Q);
+  build_rgf_upward(plan, sys, work, &up);
+  auto block = [](ZOpKind kind, const cplx* A, cplx* C, int b, cplx alpha, cplx beta, const cplx* alpha_ptr) {
+    ZBlockOp o{};
+    o.A = A; o.C = C; o.alpha_ptr = alpha_ptr; o.m = o.n = o.lda = o.ldc = b; o.kind = kind;
+    o.alpha = alpha; o.beta = beta;
+    return o;
+  };
+  {
+    std::vector<ZGemmProblem> tp, np;
+    std::vector<ZBlockOp> t0, g0, l0;
+    for (size_t k = 0; k < ns; ++k) {
+      const auto& s = sys[k];
+      RgfWork& w = work[k];
+      for (int i = 0; i < s.npl(); ++i) {
+        const int b = s.b[i];
+        tp.push_back(gp(up.op(k, i), b, w.g[i], b, i == 0 ? q[k] : t[k][i], b, b, b, b, ONE));
+        if (i > 0) tp.back().alpha_ptr = Q[k].fR;
+        np.push_back(gp(w.g[i], b, t[k][i], b, Q[k].gl[i], b, b, b, b, ONE));
+      }
+      const int b0 = s.b[0];
+      tp.push_back(gp(Q[k].gamL, b0, w.g[0], b0, t[k][0], b0, b0, b0, b0, ONE));
+      tp.back().alpha_ptr = Q[k].fL;
+      t0.push_back(block(ZOP_AXPBY, q[k], t[k][0], b0, ONE, ONE, Q[k].fR));
+      if (!Q[k].gr.empty()) g0.push_back(block(ZOP_COPY, w.g[0], Q[k].gr[0], b0, ONE, ZERO, nullptr));
+      l0.push_back(block(ZOP_AXPBY, Q[k].gl[0], Q[k].gl[0], b0, make_double2(0.0, 1.0), ZERO, nullptr));
+      G[k][0] = w.g[0];
+    }
+    plan.gemm('N', 'C', tp);
+    plan.blockops(t0);
+    plan.gemm('N', 'N', np);
+    plan.blockops(g0);
+    if (!g0.empty() && gr_final) gr_final(0);
+    plan.blockops(l0);  // G^< = i G^n
+    if (gl_final) gl_final(0);
+  }
+  auto g0 = [&](size_t k, int i) -> cplx* { return i == 0 ? work[k].g[0] : y[k][i & 1]; };
+  auto push_u = [&](int i, std::vector<ZGemmProblem>& v) {
+    for (size_t k = 0; k < ns; ++k) {
+      const auto& s = sys[k];
+      if (i + 1 >= s.npl()) continue;
+      v.push_back(gp(G[k][i], s.b[i], work[k].R[i], s.b[i], u[k], s.b[i], s.b[i], s.b[i + 1], s.b[i], MONE));
+    }
+  };
+  {
+    std::vector<ZGemmProblem> v;
+    push_u(0, v);
+    plan.gemm('N', 'N', v);
+  }
+  for (int i = 0; i + 1 < maxN; ++i) {
+    std::vector<ZGemmProblem> a, c, x;
+    std::vector<ZBlockOp> h;
+    bool any_gr = false;
+    for (size_t k = 0; k < ns; ++k) {
+      const auto& s = sys[k];
+      if (i + 1 >= s.npl()) continue;
+      RgfWork& w = work[k];
+      const int b = s.b[i], b1 = s.b[i + 1];
+      a.push_back(gp(w.L[i], b1, u[k], b, G[k][i + 1], b1, b1, b1, b, MONE, w.g[i + 1], b1, ONE));
+      a.push_back(gp(u[k], b, t[k][i + 1], b1, ub[k], b, b, b1, b1, ONE));
+      if (Q[k].t_out)
+        a.push_back(gp(g0(k, i), s.b[0], w.R[i], b, g0(k, i + 1), s.b[0], s.b[0], b1, b, MONE));
+      // gl[i] = i G^n_ii, so -G^n_ii / 2 is (i / 2) gl[i]
+      c.push_back(gp(Q[k].gl[i], b, w.L[i], b1, ub[k], b, b, b1, b, make_double2(0.0, 0.5), ub[k], b, ONE));
+      // t_{i+1} is done with: it takes n_{i+1} / 2 - L_{i+1} A
+      x.push_back(gp(w.L[i], b1, ub[k], b, t[k][i + 1], b1, b1, b1, b, MONE, Q[k].gl[i + 1], b1,
+                     make_double2(0.5, 0.0)));
+      h.push_back(block(ZOP_HERM_SUM, t[k][i + 1], Q[k].gl[i + 1], b1, make_double2(0.0, 1.0), ZERO, nullptr));
+      any_gr = any_gr || !Q[k].gr.empty();
+    }
+    plan.gemm('N', 'N', a);
+    if (any_gr && gr_final) gr_final(i + 1);
+    plan.gemm('N', 'C', c);
+    push_u(i + 1, x);
+    plan.gemm('N', 'N', x);
+    plan.blockops(h);
+    if (gl_final) gl_final(i + 1);
+  }
+  std::vector<ZGemmProblem> p1, p2;
+  std::vector<ZTraceProblemHost> tr;
+  for (size_t k = 0; k < ns; ++k) {
+    if (!Q[k].t_out) continue;
+    const auto& s = sys[k];
+    const int n = s.npl(), b0 = s.b[0], bN = s.b[n - 1];
+    p1.push_back(gp(Q[k].gamL, b0, g0(k, n - 1), b0, y[k][2], b0, b0, bN, b0, ONE));
+    p2.push_back(gp(Q[k].gamR, bN, g0(k, n - 1), b0, y[k][3], bN, bN, b0, bN, ONE));
+    ZTraceProblemHost x{};
+    x.X = y[k][2]; x.ldx = b0; x.Y = y[k][3]; x.ldy = bN; x.n = b0; x.out = Q[k].t_out;
+    tr.push_back(x);
+  }
+  plan.gemm('N', 'N', p1);
+  plan.gemm('N', 'C', p2);
+  plan.trace(tr);
 }
 
 }  // namespace negf

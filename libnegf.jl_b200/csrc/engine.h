@@ -298,9 +298,19 @@ struct TriOut {
 
 void alloc_rgf_work(Plan& plan, const TriSystem& s, RgfWork& w);
 // Upward pass (src/matinvertndiag_rgf.jl:143-162), all systems batched per layer.
-void build_rgf_upward(Plan& plan, const std::vector<TriSystem>& sys, std::vector<RgfWork>& work);
+// gn, when given, adds the upward products of a Hermitian operator to the pass's
+// own launches; for layer i of system k: before (op N, C; R_i is ready), off
+// (N, N), and after (N, C, one round later, for every layer down to 0).
+struct GnUpward {
+  virtual ~GnUpward() = default;
+  virtual void before(const TriSystem&, RgfWork&, size_t, int, std::vector<ZGemmProblem>&) {}
+  virtual void off(const TriSystem&, RgfWork&, size_t, int, std::vector<ZGemmProblem>&) = 0;
+  virtual void after(const TriSystem&, RgfWork&, size_t, int, std::vector<ZGemmProblem>&) = 0;
+};
+void build_rgf_upward(Plan& plan, const std::vector<TriSystem>& sys, std::vector<RgfWork>& work,
+                      GnUpward* gn = nullptr);
 // Downward pass (src/matinvertndiag_rgf.jl:166-182) writing the tridiagonal of
-// M^{-1}; with full_rows/full_cols the whole inverse (rgf.jl:185-199) is
+// M^{-1} (blocks below the diagonal whose output is null are not computed); with full_rows/full_cols the whole inverse (rgf.jl:185-199) is
 // written into full[s][i*npl+j] (null = skip).
 // on_final(i), when given, is called once layer i's diagonal output is final
 // for every system (in layer order).
@@ -308,16 +318,30 @@ void build_rgf_downward(Plan& plan, const std::vector<TriSystem>& sys, std::vect
                         std::vector<TriOut>& out, const std::function<void(int)>& on_final = {});
 void build_rgf_full_inverse(Plan& plan, const std::vector<TriSystem>& sys, std::vector<RgfWork>& work,
                             std::vector<std::vector<cplx*>>& full);
-// RKD passes (src/keldyshndiag.jl:221-317).  S holds the Hermitian middle
-// operator (diagonal + upper blocks) on entry and G^n on exit.
+// RGF upward and RKD passes (src/keldyshndiag.jl:221-317).  S holds the
+// Hermitian middle operator (diagonal + upper blocks) on entry and G^n on exit.
 struct HermBlocks {
   std::vector<cplx*> d, u;
   std::vector<int> ldd, ldu;
 };
-// on_final(i), when given, is called once G^n's diagonal block i is final
-// (no later step of the pass reads or writes it) for every system.
 void build_rkd(Plan& plan, const std::vector<TriSystem>& sys, std::vector<RgfWork>& work,
-               std::vector<HermBlocks>& S, const std::function<void(int)>& on_final = {});
+               std::vector<HermBlocks>& S);
+
+// G^R (optional) and G^< diagonals and the transmission (optional) of systems
+// driven by their leads only: Sigma^in = f_L Gamma_L on layer 0 and f_R Gamma_R
+// on layer N-1 (f_L, f_R: device scalars).  Includes the RGF upward pass.
+// gr_final(i) / gl_final(i) are called once layer i of that output is final.
+struct LeadSystem {
+  const cplx *gamL, *gamR;
+  const cplx *fL, *fR;
+  std::vector<cplx*> gr;    // diagonal blocks of G^R (empty: not wanted)
+  std::vector<cplx*> gl;    // diagonal blocks of G^<
+  double* t_out = nullptr;  // transmission (re, im), null: not wanted
+  cplx* v = nullptr;        // workspace of the pass
+};
+void build_lead_pass(Plan& plan, const std::vector<TriSystem>& sys, std::vector<RgfWork>& work,
+                     std::vector<LeadSystem>& Q, const std::function<void(int)>& gr_final,
+                     const std::function<void(int)>& gl_final);
 
 // Block selected inverse (selinv.cu): Block_factorization! and / or
 // Block_inverse! (src/selected_inverse.jl:9-206, mode bit 1 / bit 2) in place

@@ -150,7 +150,7 @@ struct negf_solver_s {
   int nE = 0;                               // energies of all devices
   negf_solve_opts opts{};
   std::unique_ptr<Plan> plan;
-  cplx* params = nullptr;  // [shift (nE) | f_L (nE) | f_R (nE) | i (1)]
+  cplx* params = nullptr;  // [shift (nE) | f_L (nE) | f_R (nE)]
   cplx* gr = nullptr;      // nE * sum b_i^2
   cplx* gl = nullptr;
   double* t2 = nullptr;    // 2 * nE (re, im)
@@ -184,8 +184,9 @@ size_t solver_bytes_per_energy(const negf_device_s& d, const negf_solve_opts& o)
   for (size_t i = 0; i + 1 < n; ++i) sbb += (size_t)d.b[i] * d.b[i + 1];
   size_t nb = gj_panel_width((int)mb);
   size_t c = sb2 + 2 * sbb + mb * mb + 2 * mb * nb;  // RGF work
-  if (o.want_gr) c += sb2 + 4 * mb * mb;              // G^R diagonal + rings
-  if (o.want_gl) c += sb2 + sbb + 3 * n * mb * mb;    // G^n storage + RKD scratch
+  if (o.want_gr) c += sb2;                            // G^R diagonal
+  if (o.want_gl) c += 2 * sb2 + 6 * mb * mb;          // G^n storage, t_i per layer, scratch
+  else c += 2 * mb * mb;                              // G^R ring
   if (o.want_t) c += 4 * mb * mb;
   if (d.has_S || o.sigma_per_energy) c += sb2 + 2 * sbb;  // per-energy M blocks
   if (o.sigma_per_energy) c += 2 * ((size_t)d.b.front() * d.b.front() + (size_t)d.b.back() * d.b.back());
@@ -233,13 +234,11 @@ int build_solver(negf_solver_s& S) {
   if ((int)items.size() != nE) return fail(NEGF_ERR_INVALID, "energy counts do not add up");
   S.out_total = off;
   S.per_energy = S.devs.size() == 1 ? off / (size_t)nE : 0;
-  S.params = plan.alloc_c(3 * (size_t)nE + 1);
+  S.params = plan.alloc_c(3 * (size_t)nE);
   S.info = static_cast<int*>(plan.alloc(sizeof(int) * nE));
   if (S.opts.want_gr) S.gr = plan.alloc_c(S.out_total);
   if (S.opts.want_gl) S.gl = plan.alloc_c(S.out_total);
   if (S.opts.want_t) S.t2 = static_cast<double*>(plan.alloc(sizeof(double) * 2 * nE));
-  const cplx i_unit = make_double2(0.0, 1.0);
-  NEGF_TRY_CUDA(cudaMemcpy(S.params + 3 * nE, &i_unit, sizeof(cplx), cudaMemcpyHostToDevice), "solver params");
   if (S.opts.precision != NEGF_PREC_FP64 && S.opts.precision != NEGF_PREC_MIXED)
     return fail(NEGF_ERR_INVALID, "precision must be NEGF_PREC_FP64 or NEGF_PREC_MIXED");
   for (negf_device_s* dv : S.devs) {
@@ -364,39 +363,22 @@ int build_solver(negf_solver_s& S) {
     for (int i = 0; i < d.npl; ++i) { v.push_back(base + o); o += (size_t)d.b[i] * d.b[i]; }
     return v;
   };
-  std::vector<HermBlocks> herm(nE);
   if (S.opts.want_gl) {
-    // Sigma^in = f_L Gamma_L (+) f_R Gamma_R in Hermitian storage
-    std::vector<ZBlockOp> zero, setL, addR;
+    std::vector<LeadSystem> lead(nE);
     for (int e = 0; e < nE; ++e) {
-      const negf_device_s& d = *items[e].d;
-      const int n = d.npl;
-      HermBlocks& h = herm[e];
-      h.d = out_blocks(S.gl, e);
-      for (int i = 0; i < n; ++i) h.ldd.push_back(d.b[i]);
-      for (int i = 0; i + 1 < n; ++i) {
-        h.u.push_back(plan.alloc_c((size_t)d.b[i] * d.b[i + 1]));
-        h.ldu.push_back(d.b[i]);
-      }
-      // every pass starts from Sigma^in: zero all diagonal and upper blocks
-      for (int i = 0; i < n; ++i) {
-        ZBlockOp z{}; z.C = h.d[i]; z.ldc = d.b[i]; z.m = z.n = d.b[i]; z.kind = ZOP_FILL;
-        zero.push_back(z);
-      }
-      for (int i = 0; i + 1 < n; ++i) {
-        ZBlockOp z{}; z.C = h.u[i]; z.ldc = d.b[i]; z.m = d.b[i]; z.n = d.b[i + 1]; z.kind = ZOP_FILL;
-        zero.push_back(z);
-      }
-      ZBlockOp l{}; l.A = gamL_of[e]; l.lda = d.b[0]; l.C = h.d[0]; l.ldc = d.b[0]; l.m = l.n = d.b[0];
-      l.kind = ZOP_AXPBY; l.alpha_ptr = S.params + nE + e; l.beta = make_double2(1.0, 0.0);
-      setL.push_back(l);
-      ZBlockOp r{}; r.A = gamR_of[e]; r.lda = d.b[n - 1]; r.C = h.d[n - 1]; r.ldc = d.b[n - 1];
-      r.m = r.n = d.b[n - 1]; r.kind = ZOP_AXPBY; r.alpha_ptr = S.params + 2 * nE + e; r.beta = make_double2(1.0, 0.0);
-      addR.push_back(r);
+      LeadSystem& q = lead[e];
+      q.gamL = gamL_of[e];
+      q.gamR = gamR_of[e];
+      q.fL = S.params + nE + e;
+      q.fR = S.params + 2 * nE + e;
+      if (S.opts.want_gr) q.gr = out_blocks(S.gr, e);
+      q.gl = out_blocks(S.gl, e);
+      if (S.opts.want_t) q.t_out = S.t2 + 2 * e;
     }
-    plan.blockops(zero);
-    plan.blockops(setL);
-    plan.blockops(addR);
+    build_lead_pass(plan, sys, work, lead, [&](int i) { plan.mark(kMarkGR + i); },
+                    [&](int i) { plan.mark(kMarkGL + i); });
+    NEGF_TRY_CUDA(plan.finalize(), "solver finalize");
+    return NEGF_SUCCESS;
   }
   build_rgf_upward(plan, sys, work);
   if (S.opts.want_gr) {
@@ -407,30 +389,15 @@ int build_solver(negf_solver_s& S) {
       o.d = out_blocks(S.gr, e);
       for (int i = 0; i < d.npl; ++i) o.ldd.push_back(d.b[i]);
       int mb = sys[e].maxb();
-      cplx* ring = plan.alloc_c(4 * (size_t)mb * mb);
+      cplx* ring = plan.alloc_c(2 * (size_t)mb * mb);
       for (int i = 0; i + 1 < d.npl; ++i) {
         o.u.push_back(ring + (size_t)(i % 2) * mb * mb);
-        o.l.push_back(ring + (size_t)(2 + i % 2) * mb * mb);
+        o.l.push_back(nullptr);
         o.ldu.push_back(d.b[i]);
         o.ldl.push_back(d.b[i + 1]);
       }
     }
     build_rgf_downward(plan, sys, work, out, [&](int i) { plan.mark(kMarkGR + i); });
-  }
-  if (S.opts.want_gl) {
-    // G^< = i G^n, layer by layer as soon as G^n's layer is final
-    build_rkd(plan, sys, work, herm, [&](int i) {
-      std::vector<ZBlockOp> sc;
-      for (int e = 0; e < nE; ++e) {
-        const negf_device_s& d = *items[e].d;
-        if (i >= d.npl) continue;
-        ZBlockOp o{}; o.A = herm[e].d[i]; o.lda = d.b[i]; o.C = herm[e].d[i]; o.ldc = d.b[i];
-        o.m = o.n = d.b[i]; o.kind = ZOP_AXPBY; o.alpha_ptr = S.params + 3 * nE; o.beta = make_double2(0.0, 0.0);
-        sc.push_back(o);
-      }
-      plan.blockops(sc);
-      plan.mark(kMarkGL + i);
-    });
   }
   if (S.opts.want_t) {
     // G^R_{1N} by G_{1,j} = -G_{1,j-1} R_{j-1}, G_{1,1} = g_1 (rgf.jl:169, :185-199)
@@ -509,7 +476,7 @@ int negf_zgemm_batched(char opA, char opB, int32_t nprob, const negf_zgemm_probl
       if (q.m < 0 || q.n < 0 || q.k < 0) return fail(NEGF_ERR_INVALID, "negative dimension");
       ZGemmProblem& p = v[i];
       p.A = static_cast<const cplx*>(q.A); p.B = static_cast<const cplx*>(q.B);
-      p.Cin = static_cast<const cplx*>(q.Cin); p.C = static_cast<cplx*>(q.C); p.diag_ptr = nullptr;
+      p.Cin = static_cast<const cplx*>(q.Cin); p.C = static_cast<cplx*>(q.C); p.diag_ptr = nullptr; p.alpha_ptr = nullptr;
       p.m = q.m; p.n = q.n; p.k = q.k;
       p.lda = std::max(1, q.lda); p.ldb = std::max(1, q.ldb); p.ldc = std::max(1, q.ldc);
       p.ldcin = std::max(1, q.ldcin); p.pad_ = 0;
@@ -546,7 +513,7 @@ int negf_zgemm_batched_mixed(char opA, char opB, int32_t nprob, const negf_zgemm
         return fail(NEGF_ERR_INVALID, "dimensions must be >= 0 and k <= 1024");
       ZGemmProblem& p = v[i];
       p.A = static_cast<const cplx*>(q.A); p.B = static_cast<const cplx*>(q.B);
-      p.Cin = static_cast<const cplx*>(q.Cin); p.C = static_cast<cplx*>(q.C); p.diag_ptr = nullptr;
+      p.Cin = static_cast<const cplx*>(q.Cin); p.C = static_cast<cplx*>(q.C); p.diag_ptr = nullptr; p.alpha_ptr = nullptr;
       p.m = q.m; p.n = q.n; p.k = q.k;
       p.lda = std::max(1, q.lda); p.ldb = std::max(1, q.ldb); p.ldc = std::max(1, q.ldc);
       p.ldcin = std::max(1, q.ldcin); p.pad_ = 0;
@@ -694,7 +661,7 @@ int negf_rgf(int32_t nsys, int32_t npl, const int32_t* block_sizes, void* const*
         cplx* u = pick(Gu, (size_t)s * (npl - 1) + i, i, i + 1);
         cplx* l = pick(Gl, (size_t)s * (npl - 1) + i, i + 1, i);
         if (!u) u = plan.alloc_c((size_t)t.b[i] * t.b[i + 1]);
-        if (!l) l = plan.alloc_c((size_t)t.b[i] * t.b[i + 1]);
+        if (!l && Gfull) l = plan.alloc_c((size_t)t.b[i] * t.b[i + 1]);
         o.u.push_back(u); o.ldu.push_back(t.b[i]);
         o.l.push_back(l); o.ldl.push_back(t.b[i + 1]);
       }
@@ -740,7 +707,6 @@ int negf_keldysh(int32_t nsys, int32_t npl, const int32_t* block_sizes, void* co
         herm[s].ldu.push_back(sys[s].b[i]);
       }
     }
-    build_rgf_upward(plan, sys, work);
     build_rkd(plan, sys, work, herm);
     return run_plan_sync(plan, static_cast<cudaStream_t>(stream), dinfo, nsys, "negf_keldysh");
   } catch (const std::bad_alloc&) {

@@ -48,6 +48,7 @@ struct ZGemmProblem {
   const cplx* Cin;
   cplx* C;
   const cplx* diag_ptr;  // when set, diag is read from device memory (per-energy shift)
+  const cplx* alpha_ptr;  // when set, multiplies alpha (read from device memory: per-energy factors)
   int m, n, k;
   int lda, ldb, ldc, ldcin;
   int pad_;
@@ -116,6 +117,7 @@ struct OzMmaProblem {
   cplx* C;
   const cplx* Cin;
   const cplx* diag_ptr;
+  const cplx* alpha_ptr;
   int m, n, m_pad, n_pad, k_pad, ldc, ldcin, pad_;
   cplx alpha, beta, diag;
 };
@@ -131,6 +133,7 @@ enum ZOpKind : int {
   ZOP_GAMMA = 6,       // C = i (A - A^H)   (broadening of a self-energy)
   ZOP_CTRANS_AXPBY = 7,  // C = alpha*A^H + beta*C   (A is n x m)
   ZOP_ADD_DIAG = 8,    // C[r, r] += alpha
+  ZOP_HERM_SUM = 9,    // C = alpha (A + A^H)
 };
 
 struct ZBlockOp {

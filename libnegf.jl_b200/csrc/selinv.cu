@@ -37,7 +37,7 @@ int check_device() {
 ZGemmProblem gp(const cplx* A, int lda, const cplx* B, int ldb, cplx* C, int ldc, int m, int n, int k, cplx alpha,
                 const cplx* Cin = nullptr, int ldcin = 1, cplx beta = ZERO) {
   ZGemmProblem p;
-  p.A = A; p.B = B; p.Cin = Cin; p.C = C; p.diag_ptr = nullptr;
+  p.A = A; p.B = B; p.Cin = Cin; p.C = C; p.diag_ptr = nullptr; p.alpha_ptr = nullptr;
   p.m = m; p.n = n; p.k = k;
   p.lda = std::max(1, lda); p.ldb = std::max(1, ldb); p.ldc = std::max(1, ldc); p.ldcin = std::max(1, ldcin);
   p.pad_ = 0;

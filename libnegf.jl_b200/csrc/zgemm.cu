@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(gemm::THREADS, 2)
   const bool has_ab = p.k > 0;
   const bool has_cin = (p.beta.x != 0.0 || p.beta.y != 0.0) && p.Cin != nullptr && !preload;
   const cplx dg = p.diag_ptr ? *p.diag_ptr : p.diag;
+  const cplx al = p.alpha_ptr ? cmul(p.alpha, *p.alpha_ptr) : p.alpha;
 #pragma unroll
   for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
@@ -222,8 +223,8 @@ __global__ void __launch_bounds__(gemm::THREADS, 2)
           cplx v = make_double2(0.0, 0.0);
           if (has_ab) {
             double xr = acc_re[mi][ni][e], xi = acc_im[mi][ni][e];
-            v.x = p.alpha.x * xr - p.alpha.y * xi;
-            v.y = p.alpha.x * xi + p.alpha.y * xr;
+            v.x = al.x * xr - al.y * xi;
+            v.y = al.x * xi + al.y * xr;
           }
           if (has_cin) {
             cplx ci = p.Cin[r + (size_t)c * p.ldcin];
@@ -342,6 +343,7 @@ __global__ void __launch_bounds__(gemm3m::THREADS, 1)
   const bool has_ab = p.k > 0;
   const bool has_cin = (p.beta.x != 0.0 || p.beta.y != 0.0) && p.Cin != nullptr && !preload;
   const cplx dg = p.diag_ptr ? *p.diag_ptr : p.diag;
+  const cplx al = p.alpha_ptr ? cmul(p.alpha, *p.alpha_ptr) : p.alpha;
 #pragma unroll
   for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
@@ -355,8 +357,8 @@ __global__ void __launch_bounds__(gemm3m::THREADS, 1)
           if (has_ab) {
             double xr = P1[mi][ni][e] - P2[mi][ni][e];
             double xi = P3[mi][ni][e] - P1[mi][ni][e] - P2[mi][ni][e];
-            v.x = p.alpha.x * xr - p.alpha.y * xi;
-            v.y = p.alpha.x * xi + p.alpha.y * xr;
+            v.x = al.x * xr - al.y * xi;
+            v.y = al.x * xi + al.y * xr;
           }
           if (has_cin) {
             cplx ci = p.Cin[r + (size_t)c * p.ldcin];
@@ -503,6 +505,7 @@ __global__ void __launch_bounds__(gemm_sk::THREADS, 2)
   const bool has_ab = p.k > 0;
   const bool has_cin = (p.beta.x != 0.0 || p.beta.y != 0.0) && p.Cin != nullptr && !preload;
   const cplx dg = p.diag_ptr ? *p.diag_ptr : p.diag;
+  const cplx al = p.alpha_ptr ? cmul(p.alpha, *p.alpha_ptr) : p.alpha;
 #pragma unroll
   for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
@@ -514,8 +517,8 @@ __global__ void __launch_bounds__(gemm_sk::THREADS, 2)
         if (has_ab) {
           const double xr = P1[ni][e] - P2[ni][e];
           const double xi = P3[ni][e] - P1[ni][e] - P2[ni][e];
-          v.x = p.alpha.x * xr - p.alpha.y * xi;
-          v.y = p.alpha.x * xi + p.alpha.y * xr;
+          v.x = al.x * xr - al.y * xi;
+          v.y = al.x * xi + al.y * xr;
         }
         if (has_cin) {
           const cplx ci = p.Cin[r + (size_t)c * p.ldcin];
@@ -622,7 +625,7 @@ int zgemm_tiles_smallk(int m, int n) {
 
 // True when the problem qualifies for the accumulator preload variant.
 bool zgemm_preload_ok(const ZGemmProblem& p) {
-  return p.k > 0 && p.Cin != nullptr && p.alpha.y == 0.0 && p.beta.y == 0.0 &&
+  return p.k > 0 && p.Cin != nullptr && p.alpha_ptr == nullptr && p.alpha.y == 0.0 && p.beta.y == 0.0 &&
          (p.alpha.x == 1.0 || p.alpha.x == -1.0) && (p.beta.x == 1.0 || p.beta.x == -1.0);
 }
 

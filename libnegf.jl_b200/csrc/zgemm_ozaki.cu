@@ -645,7 +645,7 @@ __global__ void __launch_bounds__(oz::THREADS, 1)
       const OzMmaProblem* pp = probs + t.prob;
       eB = pp->eB[t.nt * TN + hh * 32 + lane];
       eA = pp->eA[t.mt * TM + qd * 32 + lane];
-      a = pp->alpha;
+      a = pp->alpha_ptr ? cmul(pp->alpha, *pp->alpha_ptr) : pp->alpha;
     };
     OzTile tq{};
     if (my_tiles > 0) {
