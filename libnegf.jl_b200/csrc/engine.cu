@@ -431,12 +431,9 @@ void Plan::gemm_fp64(char opA, char opB, const std::vector<ZGemmProblem>& probs)
   int total = 0;
   double fl = 0.0;
   bool pre = true;
-  int max_k = 0;
-  for (const auto& p : probs)
-    if (zgemm_tiles(p.m, p.n) > 0) max_k = std::max(max_k, p.k);
-  const bool small = zgemm_smallk_ok(gemm_form_, max_k);
+  const int form = zgemm_choose_form(gemm_form_, probs.data(), (int)probs.size());
   for (const auto& p : probs) {
-    int t = small ? zgemm_tiles_smallk(p.m, p.n) : zgemm_tiles(p.m, p.n);
+    int t = zgemm_tiles_form(form, p.m, p.n);
     if (t == 0) continue;
     v.push_back(p);
     starts.push_back(total);
@@ -449,8 +446,8 @@ void Plan::gemm_fp64(char opA, char opB, const std::vector<ZGemmProblem>& probs)
   s.kind = Step::GEMM;
   s.opA = opA;
   s.opB = opB;
-  s.preload = pre;
-  s.form = small ? 3 : gemm_form_;
+  s.preload = pre && form == 1;
+  s.form = form;
   s.uniform_tiles = total / (int)v.size();
   if ((long long)s.uniform_tiles * (long long)v.size() != total) s.uniform_tiles = 0;
   for (size_t i = 1; i < starts.size() && s.uniform_tiles; ++i)
@@ -647,7 +644,7 @@ cudaError_t Plan::finalize() {
   std::set<std::pair<char, char>> ops;
   size_t max_smem = 0, lu_smem = 0, tri_smem = 0;
   for (const auto& s : steps) {
-    if (s.kind == Step::GEMM && s.form != 4) ops.insert({s.opA, s.opB});
+    if (s.kind == Step::GEMM && s.form == 1) ops.insert({s.opA, s.opB});
     if (s.kind == Step::GJ_PANEL) max_smem = std::max(max_smem, s.smem);
     if (s.kind == Step::LU_PANEL) lu_smem = std::max(lu_smem, s.smem);
     if (s.kind == Step::TRI_DIAG) tri_smem = std::max(tri_smem, s.smem);

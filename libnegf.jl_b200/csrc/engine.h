@@ -27,11 +27,10 @@ cudaError_t launch_zgemm_batched_ex(char opA, char opB, bool preload, const ZGem
                                     int form = 0, int uniform_tiles = 0);
 bool zgemm_preload_ok(const ZGemmProblem& p);
 int zgemm_tiles(int m, int n);
-// small-K 3M kernel (32 x 64 tiles, two CTAs per SM) for steps with every
-// k <= 32 in the 3M form; a step using it carries form 3 and counts its tiles
-// with zgemm_tiles_smallk
-bool zgemm_smallk_ok(int form, int max_k);
-int zgemm_tiles_smallk(int m, int n);
+// the kernel (step form) of a list of problems under the plan's GEMM form, and
+// its tiles of a problem
+int zgemm_choose_form(int form, const ZGemmProblem* probs, int nprob);
+int zgemm_tiles_form(int form, int m, int n);
 size_t zgemm_smem_bytes();
 cudaError_t zgemm_prepare(char opA, char opB);
 size_t zgj_panel_smem_bytes(int n, int nb);
@@ -143,7 +142,7 @@ struct Step {
   int count = 0, total_tiles = 0, max_m = 0, max_n = 0;
   int k0 = 0, nb = 0, blocked = 0;
   bool preload = false;  // GEMM: accumulators start from Cin (all problems alpha, beta = +-1)
-  int form = 0;          // GEMM: 0 default, 1 four real products, 2 3M, 3 small-K 3M, 4 Gauss-Jordan update; OZ_MMA: digit pairs (34 or 28)
+  int form = 0;          // GEMM: 1 four real products, 4 Gauss-Jordan update, 5 / 6 3M (zgemm_choose_form); OZ_MMA: digit pairs (34 or 28)
   int uniform_tiles = 0; // GEMM: tiles of every problem when all have the same count, else 0
   size_t smem = 0;
   double flops = 0.0;    // real flops of the step (8mnk per complex GEMM)
