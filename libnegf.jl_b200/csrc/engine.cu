@@ -431,7 +431,7 @@ void Plan::gemm_fp64(char opA, char opB, const std::vector<ZGemmProblem>& probs)
   int total = 0;
   double fl = 0.0;
   bool pre = true;
-  const int form = zgemm_choose_form(gemm_form_, probs.data(), (int)probs.size());
+  const int form = zgemm_choose_form(gemm_form_, probs.data(), (int)probs.size(), fixed_order_);
   for (const auto& p : probs) {
     int t = zgemm_tiles_form(form, p.m, p.n);
     if (t == 0) continue;

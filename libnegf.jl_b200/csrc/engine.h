@@ -29,7 +29,7 @@ bool zgemm_preload_ok(const ZGemmProblem& p);
 int zgemm_tiles(int m, int n);
 // the kernel (step form) of a list of problems under the plan's GEMM form, and
 // its tiles of a problem
-int zgemm_choose_form(int form, const ZGemmProblem* probs, int nprob);
+int zgemm_choose_form(int form, const ZGemmProblem* probs, int nprob, bool fixed_order);
 int zgemm_tiles_form(int form, int m, int n);
 size_t zgemm_smem_bytes();
 cudaError_t zgemm_prepare(char opA, char opB);
@@ -175,6 +175,9 @@ class Plan {
   // schedule knobs: FP64 GEMM form (0 default, 1 four products, 2 3M) and the
   // Gauss-Jordan panel width for blocks > 112 (0 default)
   void set_schedule(int gemm_form, int gj_nb) { gemm_form_ = gemm_form; gj_nb_ = gj_nb; }
+  // FP64 products add in an order that does not depend on the other problems of
+  // their step: a system's results are the same whatever batch it is solved in
+  void set_fixed_order(bool on) { fixed_order_ = on; }
   // Gauss-Jordan rank-nb updates of a mixed plan: 1 FP64 DMMA products, 2
   // INT8 digit products with 34 pairs (as accurate as FP64 products), 0 the
   // default (1: at 256 x 32 layers both take the same time per pass, and the
@@ -232,7 +235,7 @@ class Plan {
   cudaGraph_t graph_ = nullptr;
   cudaGraphExec_t gexec_ = nullptr;
   cudaStream_t graph_stream_ = nullptr;
-  bool mixed_ = false;
+  bool mixed_ = false, fixed_order_ = false;
   int oz_pairs_ = 34;
   int gemm_form_ = 0, gj_nb_ = 0, gj_update_ = 0;
   int* err_ = nullptr;            // tensor-core wait time-out flag (device int)

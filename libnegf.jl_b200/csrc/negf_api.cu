@@ -260,6 +260,7 @@ int build_solver(negf_solver_s& S) {
         return fail(NEGF_ERR_INVALID, "gj_nb too wide for the block size (shared memory)");
   if (S.opts.gj_update < 0 || S.opts.gj_update > 2) return fail(NEGF_ERR_INVALID, "gj_update must be 0, 1 or 2");
   plan.set_schedule(S.opts.gemm_form, S.opts.gj_nb);
+  plan.set_fixed_order(true);  // chunks, batches and server groups of any size agree
   plan.set_gj_update(S.opts.gj_update);
 
   const bool sig_e = S.opts.sigma_per_energy != 0;
@@ -1286,6 +1287,7 @@ int negf_device_selected_inverse(negf_device_t dev, int32_t nE, const double* en
       // errors more than RGF does: FP64-grade products (34 digit pairs) there
       plan.set_mixed(mixed, method == 0 ? 28 : 34);
       plan.set_schedule(opts->gemm_form, opts->gj_nb);
+      plan.set_fixed_order(true);
       plan.set_gj_update(opts->gj_update);
       int* dinfo = static_cast<int*>(plan.alloc(sizeof(int) * (size_t)cnt * n));
       // output blocks of this chunk: the caller's device buffers, or plan memory

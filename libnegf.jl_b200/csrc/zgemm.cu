@@ -472,9 +472,12 @@ int zgemm_tiles_form(int form, int m, int n) {
 // The kernel of a step: the four-product one for form 1 (or by NEGF_ZGEMM=4m),
 // else 3M in 32 x 32 tiles, in 16 x 16 tiles when there are fewer than 96 of the
 // former: a CTA's time is then the step's (one 256 product, 64 tiles: 17.0 against
-// 10.9 us; two, 128 tiles: 17.7 against 18.7 us).
-int zgemm_choose_form(int form, const ZGemmProblem* probs, int nprob) {
+// 10.9 us; two, 128 tiles: 17.7 against 18.7 us).  The 16 x 16 form adds its K
+// slabs in another order, so fixed_order (results that do not depend on what else
+// is in the batch) keeps to 32 x 32.
+int zgemm_choose_form(int form, const ZGemmProblem* probs, int nprob, bool fixed_order) {
   if (form == 1 || (form == 0 && !use_3m())) return 1;
+  if (fixed_order) return kFormTile32;
   long long tiles = 0;
   for (int i = 0; i < nprob; ++i) tiles += zgemm_tiles_form(kFormTile32, probs[i].m, probs[i].n);
   return tiles < 96 ? kFormTile16 : kFormTile32;
