@@ -156,8 +156,9 @@ class Plan {
   Plan(const Plan&) = delete;
   Plan& operator=(const Plan&) = delete;
 
-  // device memory owned by the plan (workspace); zero-initialised, 256-byte
-  // aligned, sub-allocated from a few large chunks
+  // device memory owned by the plan (workspace); zero-initialised by finalize
+  // (nothing may be written to it before), 256-byte aligned, sub-allocated
+  // from a few large chunks
   void* alloc(size_t bytes);
   cplx* alloc_c(size_t n) { return static_cast<cplx*>(alloc(n * sizeof(cplx))); }
 
@@ -194,7 +195,10 @@ class Plan {
   void getrf(const std::vector<LuSpec>& specs);
   void trtri(const std::vector<TriSpec>& specs, bool upper);
 
+  // Uploads the descriptors, zeroes the workspace and sets kernel attributes:
+  // in order on `stream` (run calls it), or, without one, complete on return.
   cudaError_t finalize();
+  cudaError_t finalize(cudaStream_t stream);
   // Records a plan-owned event on s after work that uses the plan's memory
   // (every run does it; callers add it after their own uploads outside a
   // run).  The destructor waits for these events before the chunks are
@@ -223,9 +227,11 @@ class Plan {
   cudaError_t launch_step(const Step& s, const unsigned char* base, cudaStream_t stream);
   size_t push_bytes(const void* p, size_t n);
   void* raw_alloc(size_t bytes);
+  void* take_chunk(size_t bytes);
   std::vector<unsigned char> blob_;
   void* dblob_ = nullptr;
   std::vector<std::pair<void*, size_t>> owned_;  // chunks and their sizes
+  std::vector<std::pair<void*, size_t>> to_zero_;  // chunks that finalize zeroes
   std::vector<std::pair<cudaStream_t, cudaEvent_t>> fences_;  // last use of the memory per stream (fence)
   size_t owned_bytes_ = 0;
   std::vector<std::pair<size_t, int>> marks_;

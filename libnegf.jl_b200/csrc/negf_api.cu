@@ -44,12 +44,11 @@ inline cplx c2(const double* v) { return make_double2(v[0], v[1]); }
 int run_plan_sync(Plan& plan, cudaStream_t st, int* dinfo, int nsys, const char* what) {
   cudaError_t e = plan.run(st, false);
   if (e != cudaSuccess) return cuda_fail(e, what);
-  e = cudaStreamSynchronize(st);
+  std::vector<int> info(dinfo ? nsys : 0);
+  if (dinfo) e = cudaMemcpyAsync(info.data(), dinfo, sizeof(int) * nsys, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(e, what);
   if (dinfo) {
-    std::vector<int> info(nsys);
-    e = cudaMemcpy(info.data(), dinfo, sizeof(int) * nsys, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(e, what);
     for (int s = 0; s < nsys; ++s)
       if (info[s] != 0) {
         char buf[160];
@@ -611,10 +610,10 @@ int negf_zinv_batched(int32_t nprob, const int32_t* n, void* const* A, const int
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaError_t e = plan.run(st, false);
     if (e != cudaSuccess) return cuda_fail(e, "negf_zinv_batched");
-    NEGF_TRY_CUDA(cudaStreamSynchronize(st), "negf_zinv_batched");
     std::vector<int> h(std::max(1, nprob));
-    NEGF_TRY_CUDA(cudaMemcpy(h.data(), dinfo, sizeof(int) * std::max(1, nprob), cudaMemcpyDeviceToHost),
+    NEGF_TRY_CUDA(cudaMemcpyAsync(h.data(), dinfo, sizeof(int) * std::max(1, nprob), cudaMemcpyDeviceToHost, st),
                   "negf_zinv_batched");
+    NEGF_TRY_CUDA(cudaStreamSynchronize(st), "negf_zinv_batched");
     int bad = -1;
     for (int i = 0; i < nprob; ++i) {
       if (info) info[i] = h[i];

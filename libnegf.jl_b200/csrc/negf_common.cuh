@@ -6,11 +6,25 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 
 namespace negf {
 
 using cplx = double2;
+
+// Marks the devices on which a set-up (kernel attributes) has been done; two
+// threads that meet do it twice, which is harmless.
+class PerDevice {
+ public:
+  bool done(int dev) const { return dev >= 0 && dev < 64 && ((mask_.load() >> dev) & 1); }
+  void set(int dev) {
+    if (dev >= 0 && dev < 64) mask_.fetch_or(1ull << dev);
+  }
+
+ private:
+  std::atomic<unsigned long long> mask_{0};
+};
 
 __host__ __device__ inline cplx cmake(double r, double i) { return make_double2(r, i); }
 __host__ __device__ inline cplx cadd(cplx a, cplx b) { return make_double2(a.x + b.x, a.y + b.y); }

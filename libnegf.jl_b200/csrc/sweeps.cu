@@ -61,12 +61,11 @@ ZBlockOp copy_op(const cplx* A, int lda, cplx* C, int ldc, int m, int n) {
 int run_sync(Plan& plan, cudaStream_t st, int* dinfo, int nsys, const char* what) {
   cudaError_t e = plan.run(st, false);
   if (e != cudaSuccess) return cuda_fail(e, what);
-  e = cudaStreamSynchronize(st);
+  std::vector<int> info(dinfo ? nsys : 0);
+  if (dinfo) e = cudaMemcpyAsync(info.data(), dinfo, sizeof(int) * nsys, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(e, what);
   if (dinfo) {
-    std::vector<int> info(nsys);
-    e = cudaMemcpy(info.data(), dinfo, sizeof(int) * nsys, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(e, what);
     for (int s = 0; s < nsys; ++s)
       if (info[s]) {
         char buf[160];

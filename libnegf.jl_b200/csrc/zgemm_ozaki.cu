@@ -1006,6 +1006,10 @@ static_assert(split1_smem(128) <= kSplit1SmemMax && split1_smem(256) <= kSplit1S
               "single-read split staging");
 
 cudaError_t ozaki_prepare() {
+  static PerDevice set;
+  int dev = 0;
+  if (cudaError_t e = cudaGetDevice(&dev)) return e;
+  if (set.done(dev)) return cudaSuccess;
   // the register split of the product kernel assumes the launch allocates
   // exactly REGS_LAUNCH registers per thread; with fewer, setmaxnreg.inc of
   // the drain warps could never be satisfied, so such a build is refused
@@ -1031,6 +1035,7 @@ cudaError_t ozaki_prepare() {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(ozaki_split1_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kSplit1SmemMax);
+  if (e == cudaSuccess) set.set(dev);
   return e;
 }
 

@@ -516,10 +516,13 @@ cudaError_t zgj_prepare(size_t smem) {
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&mx, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
   if (smem > (size_t)mx) return cudaErrorInvalidValue;
+  static PerDevice set;
+  if (set.done(dev)) return cudaSuccess;
   for (const void* f : {(const void*)zgj_panel_kernel<128, 1>, (const void*)zgj_panel_kernel<256, 1>,
                         (const void*)zgj_panel_kernel<256, 2>, (const void*)zgj_panel_kernel<256, 4>,
                         (const void*)zgj_update_kernel<16>, (const void*)zgj_update_kernel<32>})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+  if (e == cudaSuccess) set.set(dev);
   return e;
 }
 
