@@ -96,16 +96,16 @@ __device__ __forceinline__ unsigned gj_key(double v, int row) {
 //    the slab take the rank-8 update on the FP64 tensor path (16 x 8 tiles, k =
 //    8, four real products): W += S Bb, and W = S Bb at the pivot rows (the
 //    form W += (S - E_P) Bb would lose digits where |S| is far below 1).
-// What bounds it: the latency of a column (about 900 cycles with four warps,
-// 1200 with eight: two reduction rounds, one barrier, one reciprocal, and some
-// 250 instructions per warp) and the FP64 pipe of one SM in the rank-8 updates.
-// Eight columns keep a row in 32 registers; wider sub-panels do more of the
-// n w^2 work in the latency-bound form, narrower ones add update passes over
-// shared memory.  A 256 x 32 panel takes 44 us (104 us with the whole slab in
-// registers and one rank-1 step per column), a whole 64 x 64 inversion 63 us
-// (192 us for 64 of them before), 100 x 100 131 us (627 us).
+// What bounds it: the latency of a column (750 cycles with one warp of rows, 830
+// with four, 1040 with eight: two reduction rounds, a barrier of the warps with
+// rows, one reciprocal, and some 250 instructions per warp) and the FP64 pipe of
+// one SM in the rank-8 updates.  Eight columns keep a row in 32 registers; wider
+// sub-panels do more of the n w^2 work in the latency-bound form, narrower ones
+// add update passes over shared memory.  A 256 x 32 panel takes 40 us (104 us
+// with the whole slab in registers and one rank-1 step per column), a whole 64 x
+// 64 inversion 57 us (192 us for 64 of them before), 100 x 100 117 us (627 us).
 template <int T, int RT>
-__global__ void __launch_bounds__(T)
+__global__ void __launch_bounds__(T, 1)
     zgj_panel_kernel(const ZInvProblem* __restrict__ probs, GjPanelArgs args) {
   using gj::SW;
   const ZInvProblem p = probs[blockIdx.x];
@@ -122,7 +122,8 @@ __global__ void __launch_bounds__(T)
   cplx* slot = Bb + (size_t)SW * SW * wt;             // [2][NW][SW] candidate rows
   uint4* part = reinterpret_cast<uint4*>(slot + 2 * NW * SW);  // [2][NW] candidate keys
   int* sh_piv = reinterpret_cast<int*>(part + 2 * NW / 4);     // w
-  uint8_t* at = reinterpret_cast<uint8_t*>(sh_piv + w);         // n: the sub-panel whose pivot row a row is
+  int* sh_dead = sh_piv + w;
+  uint8_t* at = reinterpret_cast<uint8_t*>(sh_dead + 1);        // n: the sub-panel whose pivot row a row is
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int j = warp; j < w; j += NW)
@@ -135,11 +136,15 @@ __global__ void __launch_bounds__(T)
   }
   for (int c = tid; c < w; c += T) sh_piv[c] = 0;  // valid row indices even if the column loop stops early
   for (int r = tid; r < n; r += T) at[r] = 255;
+  if (tid < 2 * NW) reinterpret_cast<unsigned*>(part)[tid] = 0u;
   gj_cp_wait();
   __syncthreads();
 
-  const bool active = warp * 32 < n;  // warps without rows only take part in the barriers and the updates
-  bool dead = false;  // a column without a candidate row: the host reports the info code
+  // warps without rows only take part in the rank-8 updates
+  const int pw = min(NW, (n + 31) / 32);
+  const bool active = warp < pw;
+  if (tid == 0) *sh_dead = 0;  // a column without a candidate row: the host reports the info code
+  bool dead = false;
   for (int s0 = 0; s0 < w && !dead; s0 += SW) {
     const int sw = min(SW, w - s0);
     cplx a[RT][SW];
@@ -171,7 +176,7 @@ __global__ void __launch_bounds__(T)
     // register column q - 1 and the finished column to the last one, so the loop
     // is not unrolled.
 #pragma unroll 1
-    for (int j = 0; j < sw; ++j) {
+    for (int j = 0; active && j < sw; ++j) {
       const int buf = (j & 1) * NW;
       if (lane == 0) reinterpret_cast<unsigned*>(part)[buf + warp] = wkey;
       if (key == wkey && key != 0u) {
@@ -183,27 +188,35 @@ __global__ void __launch_bounds__(T)
             for (int q = 1; q < SW; ++q) ws[q] = a[k][q];
         ws[0] = gj_pivot_inv(cand);
       }
-      __syncthreads();
-      unsigned best = 0;
+      unsigned best = wkey;
+      if (pw == 1) {
+        __syncwarp();
+      } else {
+        asm volatile("bar.sync 1, %0;" ::"r"(pw * 32) : "memory");  // the warps with rows
 #pragma unroll
-      for (int q = 0; q < NW / 4; ++q) {
-        const uint4 x = part[buf / 4 + q];
-        best = max(max(best, max(x.x, x.y)), max(x.z, x.w));
+        for (int q = 0; q < NW / 4; ++q) {
+          const uint4 x = part[buf / 4 + q];  // zero for the warps without rows
+          best = max(max(best, max(x.x, x.y)), max(x.z, x.w));
+        }
       }
       const int pr = 1023 - (int)(best & 1023u);
-      if (best == 0u) {  // no candidate row (uniform)
-        dead = true;
-        if (tid == 0) sh_piv[s0 + j] = -1;
-        if (tid == 0 && p.info) atomicCAS(p.info, 0, k0 + s0 + j + 1);
-        break;
+      if (best < 2048u) {  // no candidate row, or one whose leading bits are zero (uniform)
+        if (best == 0u) {
+          if (tid == 0) {
+            *sh_dead = 1;
+            sh_piv[s0 + j] = -1;
+            if (p.info) atomicCAS(p.info, 0, k0 + s0 + j + 1);
+          }
+          break;
+        }
+        const cplx x = slot[(buf + ((pr % T) >> 5)) * SW];  // 0 for a zero pivot
+        if (tid == 0 && p.info && x.x == 0.0 && x.y == 0.0) atomicCAS(p.info, 0, k0 + s0 + j + 1);
       }
       const cplx* row = slot + (buf + ((pr % T) >> 5)) * SW;
-      if (tid == 0) {
+      if (tid == pw * 32 - 1) {
         sh_piv[s0 + j] = pr;
         at[pr] = (uint8_t)(s0 / SW);
-        if (p.info && row[0].x == 0.0 && row[0].y == 0.0) atomicCAS(p.info, 0, k0 + s0 + j + 1);  // zero pivot
       }
-      if (!active) continue;
       // row r -= f row(pivot) with f = a[r][j] / pivot; the pivot row itself is
       // 0 - (-1/pivot) row(pivot)
       const cplx pv = row[0];
@@ -237,6 +250,7 @@ __global__ void __launch_bounds__(T)
         if (r < n && j >= 0) S[(size_t)(s0 + j) * ldw + r] = a[k][q];
       }
     __syncthreads();
+    dead = *sh_dead != 0;
     if (dead || wt == 1) continue;
     // the pivot rows in the other columns (unused k of a last, narrower tile: zero)
     for (int i = tid; i < SW * SW * wt; i += T) {
@@ -471,14 +485,15 @@ __global__ void zgj_unpermute_kernel(const ZInvProblem* __restrict__ probs) {
 size_t zgj_panel_smem_bytes(int n, int nb) {
   const size_t w = nb < n ? nb : n, w8 = (w + gj::SW - 1) / gj::SW * gj::SW;
   size_t b = (size_t)(n | 1) * w8 * sizeof(cplx) + w8 * gj::SW * sizeof(cplx);
-  b += 2 * 8 * (gj::SW * sizeof(cplx) + sizeof(unsigned)) + w * sizeof(int) + n;
+  b += 2 * 8 * (gj::SW * sizeof(cplx) + sizeof(unsigned)) + (w + 1) * sizeof(int) + n;
   return (b + 15) & ~size_t(15);
 }
 
 // One thread per row up to 256 rows, then two and four rows per thread.  Up to
 // 128 rows four warps, whose barriers are cheaper and whose CTAs share an SM --
 // except a whole matrix above 64, whose rank-8 updates want eight warps (n =
-// 100: 131 us against 162 us; n = 64: 64 us both, 592 matrices 152 against 137).
+// 100: 131 us against 162 us; n = 64: 62 against 58 us, 592 matrices 149 against
+// 130).
 cudaError_t launch_zgj_panel(const ZInvProblem* probs_dev, int nprob, int k0, int nb, int blocked, size_t smem,
                              cudaStream_t stream, int max_n) {
   if (nprob <= 0) return cudaSuccess;
