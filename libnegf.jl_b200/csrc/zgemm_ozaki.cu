@@ -96,90 +96,115 @@ __device__ __forceinline__ double oz_i2d(uint32_t x) {
 
 __device__ __forceinline__ uint32_t oz_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// rint(y) for |y| < 2^54 as an int64, on the FP64 add pipe: with M = 2^52 +
-// 2^51, the low word of t + M is rint(t) for |t| < 2^31; y is taken in two
-// 27-bit halves (both steps exact but the final rounding of the low half)
-__device__ __forceinline__ long long oz_rint54(double y) {
+// rint(t 2^27) + c for |t| < 2^27, on the FP64 add pipe: with M = 2^52 + 2^51,
+// the low word of x + M is rint(x) for |x| < 2^31; t is taken as its integer part
+// and 27 further bits (both steps exact but the final rounding)
+__device__ __forceinline__ long long oz_rint54(double t, long long c) {
   constexpr double M = 6755399441055744.0;  // 2^52 + 2^51
-  const double t = y * 0x1p-27;
-  const double th = (t + M) - M;            // rint(t), |th| <= 2^27
-  const int hi = __double2loint(t + M);
-  const double yl = fma(-th, 0x1p27, y);    // exact, |yl| <= 2^26
-  const int lo = __double2loint(yl + M);
-  return ((long long)hi << 27) + lo;
+  const double u = t + M;
+  const double r = t - (u - M);             // exact, |r| <= 1/2
+  return (long long)__double2loint(u) * (1LL << 27) + ((long long)__double2loint(fma(r, 0x1p27, M)) + c);
 }
 
-// gather byte `bb` of four words into one word (element j -> byte j)
-__device__ __forceinline__ uint32_t oz_gather(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, uint32_t bb) {
-  const uint32_t sel = bb | ((bb + 4u) << 4);
-  return __byte_perm(__byte_perm(w0, w1, sel), __byte_perm(w2, w3, sel), 0x5410);
+// 4 x 4 byte transpose: word i of the result holds byte i of w0, w1, w2, w3
+__device__ __forceinline__ void oz_transpose(const uint32_t (&w)[4], uint32_t (&o)[4]) {
+  const uint32_t a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140);
+  const uint32_t c = __byte_perm(w[0], w[1], 0x7362), d = __byte_perm(w[2], w[3], 0x7362);
+  o[0] = __byte_perm(a, b, 0x5410);
+  o[1] = __byte_perm(a, b, 0x7632);
+  o[2] = __byte_perm(c, d, 0x5410);
+  o[3] = __byte_perm(c, d, 0x7632);
 }
 
 // Digit store of one lane: 4 consecutive k of row `grow` in each K half of
 // chunk c (row[16h + j] = element c*32 + 16h + 4kq + j, in shared memory), as
 // 3 real operands x 7 byte slices in the product kernel's core-matrix layout.
 // A warp whose lanes are (row % 8) * 4 + kq covers one 128-byte core matrix
-// per store.
+// per store.  The kernel is bound by its instructions as much as by memory, so
+// the scale goes straight to the integer part (f = 2^(27 - e); TWO: as f f2,
+// for rows below 2^-990), the bytes are transposed four elements at a time and
+// the offsets of the slices are compile-time ones.
+// Left operand (128-row tiles): slice i at i * 4096, K halves 2048 apart; right
+// operand (64-row tiles): the seven slices form one 448-row K-major matrix (row
+// = 64 i + r), so slice i starts at i * 1024, K halves 7168 apart.
+template <bool LEFT, bool TWO>
 __device__ __forceinline__ void oz_store_digits(const OzSplitProblem& q, int grow, int kq, int c, const cplx* row,
-                                                double f1, double fi, double f2) {
-  const int TR = q.tile_rows;
+                                                double f, double fi, double f2) {
+  constexpr int TR = LEFT ? oz::TM : oz::TN;
+  constexpr int SLICE = LEFT ? oz::TM * oz::KC : oz::TN * 16, HALF = LEFT ? oz::TM * 16 : oz::S * oz::TN * 16;
+  constexpr int BLOCK = oz::S * TR * oz::KC;
   const int t = grow / TR, rt = grow % TR;
   const int kch = q.k_pad / oz::KC;
-  // left operand (128-row tiles): slice i at i * 4096, K halves 2048 apart;
-  // right operand (64-row tiles): the seven slices form one 448-row K-major
-  // matrix (row = 64 i + r), so slice i starts at i * 1024, K halves 7168 apart
-  const size_t slice = TR == oz::TM ? (size_t)TR * oz::KC : (size_t)TR * 16;
-  const size_t half = TR == oz::TM ? (size_t)TR * 16 : (size_t)oz::S * TR * 16;
-  const size_t block = (size_t)oz::S * TR * oz::KC;
-  const int ntiles = q.rows_pad / TR;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  const size_t op = (size_t)(q.rows_pad / TR) * kch * BLOCK;  // one real operand
+  uint8_t* base = reinterpret_cast<uint8_t*>(q.slices) + ((size_t)t * kch + c) * BLOCK + (rt >> 3) * 128 +
+                  (rt & 7) * 16 + 4 * kq;
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h, base += HALF, row += 16) {
     // offset fixed-point values x + C6 of re, im and re + im of 4 consecutive
     // k: byte 6 is the top digit, bytes 5..0 are the lower digits + 128
-    uint32_t lo[3][4], hi[3][4];
+    long long xr[4], xi[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const cplx v = row[16 * h + j];
-      const long long xr = oz_rint54(v.x * f1 * f2);
-      const long long xi = oz_rint54(v.y * fi * f2);
-      const long long x3[3] = {xr + oz::C6, xi + oz::C6, xr + xi + oz::C6};
-#pragma unroll
-      for (int p = 0; p < 3; ++p) {
-        lo[p][j] = (uint32_t)x3[p];
-        hi[p][j] = (uint32_t)((unsigned long long)x3[p] >> 32);
-      }
+      const cplx v = row[j];
+      xr[j] = oz_rint54(TWO ? v.x * f * f2 : v.x * f, oz::C6);
+      xi[j] = oz_rint54(TWO ? v.y * fi * f2 : v.y * fi, oz::C6);
     }
-    const size_t inrow = (size_t)h * half + (size_t)(rt >> 3) * 128 + (rt & 7) * 16 + 4 * kq;
+    uint8_t* o = base;
 #pragma unroll
-    for (int p = 0; p < 3; ++p) {
-      uint8_t* base = reinterpret_cast<uint8_t*>(q.slices) + ((size_t)(p * ntiles + t) * kch + c) * block + inrow;
+    for (int p = 0; p < 3; ++p, o += op) {
+      uint32_t lo[4], hi[4], l[4], g[4];
 #pragma unroll
-      for (int i = 0; i < oz::S; ++i) {
-        const int bi = oz::S - 1 - i;  // byte of digit slice i
-        uint32_t w = bi < 4 ? oz_gather(lo[p][0], lo[p][1], lo[p][2], lo[p][3], bi)
-                            : oz_gather(hi[p][0], hi[p][1], hi[p][2], hi[p][3], bi - 4);
-        if (i > 0) w ^= 0x80808080u;  // lower digits: byte - 128
-        *reinterpret_cast<uint32_t*>(base + i * slice) = w;
+      for (int j = 0; j < 4; ++j) {
+        const long long x = p == 0 ? xr[j] : p == 1 ? xi[j] : xr[j] + (xi[j] - oz::C6);
+        lo[j] = (uint32_t)x;
+        hi[j] = (uint32_t)((unsigned long long)x >> 32);
       }
+      oz_transpose(lo, l);
+      oz_transpose(hi, g);
+      // digit slice i is byte 6 - i; lower digits: byte - 128
+      *reinterpret_cast<uint32_t*>(o) = g[2];
+      *reinterpret_cast<uint32_t*>(o + SLICE) = g[1] ^ 0x80808080u;
+      *reinterpret_cast<uint32_t*>(o + 2 * SLICE) = g[0] ^ 0x80808080u;
+#pragma unroll
+      for (int i = 3; i < oz::S; ++i) *reinterpret_cast<uint32_t*>(o + i * SLICE) = l[6 - i] ^ 0x80808080u;
     }
   }
 }
 
-// Scale factors of a row with exponent e: x = rint(v 2^(54 - e)) through two
-// exact power-of-two factors (|x| <= 2^54); fi carries the conjugation.
-__device__ __forceinline__ void oz_row_factors(int e, int conj, double& f1, double& fi, double& f2) {
-  const int sh = 54 - e;
-  f1 = ldexp(1.0, sh / 2);
-  f2 = ldexp(1.0, sh - sh / 2);
-  fi = conj ? -f1 : f1;
+// Scale factors of a row with exponent e: 2^(27 - e) as f f2 (f2 = 1 unless the
+// row lies below 2^-990); fi carries the conjugation.
+__device__ __forceinline__ void oz_row_factors(int e, int conj, double& f, double& fi, double& f2) {
+  const int sh = 27 - e, s1 = min(sh, 1016);
+  f = ldexp(1.0, s1);
+  f2 = ldexp(1.0, sh - s1);
+  fi = conj ? -f : f;
+}
+
+__device__ __forceinline__ void oz_digits(const OzSplitProblem& q, int e, int grow, int kq, int c, const cplx* row) {
+  double f, fi, f2;
+  oz_row_factors(e, q.conj, f, fi, f2);
+  const bool two = __any_sync(0xffffffffu, f2 != 1.0);
+  if (q.tile_rows == oz::TM) {
+    if (two) oz_store_digits<true, true>(q, grow, kq, c, row, f, fi, f2);
+    else oz_store_digits<true, false>(q, grow, kq, c, row, f, fi, f2);
+  } else {
+    if (two) oz_store_digits<false, true>(q, grow, kq, c, row, f, fi, f2);
+    else oz_store_digits<false, false>(q, grow, kq, c, row, f, fi, f2);
+  }
 }
 
 // Single-read split: the CTA stages R whole rows (all k_pad columns) in shared
 // memory once, takes the row maxima there and writes the digits from there,
-// so each operand element is read from memory once.  For k_pad <= 512
-// (R = 32, 16, 8 rows for k_pad <= 128, 256, 512; <= 66 KB of staging).
+// so each operand element is read from memory once.  For k_pad <= 512 (R = 16
+// rows for k_pad <= 128, else 8; 33 KB of staging and five CTAs per SM up to
+// k_pad = 256).  Bound: HBM (16 bytes read and 21 written per element, 4.8 TB/s
+// at 64 x 256 x 256, three quarters of a copy's rate: the writes are 128-byte
+// pieces) and its instructions (three quarters of those of 32-bit slice words
+// gathered byte by byte and a scale applied before the integer split).  Keeping
+// the next rows in flight in a second buffer was slower (27.6 against 23.3 ms
+// per pass of 64 energies of 32 x 256): a third of the warps.
 template <int R>
-__global__ void __launch_bounds__(256, 3) ozaki_split1_kernel(const OzSplitProblem* __restrict__ probs, int ldt) {
+__global__ void __launch_bounds__(256, 5) ozaki_split1_kernel(const OzSplitProblem* __restrict__ probs, int ldt) {
   const OzSplitProblem q = probs[blockIdx.y];
   const int r0 = blockIdx.x * R;
   if (r0 >= q.rows_pad) return;
@@ -234,9 +259,7 @@ __global__ void __launch_bounds__(256, 3) ozaki_split1_kernel(const OzSplitProbl
   for (int item = warp; item < (R / 8) * kch; item += 8) {
     const int g = item % (R / 8), c = item / (R / 8);
     const int rl = g * 8 + (lane >> 2);
-    double f1, fi, f2;
-    oz_row_factors(sh_e[rl], q.conj, f1, fi, f2);
-    oz_store_digits(q, r0 + rl, kq, c, tile + (size_t)rl * ldt + c * oz::KC + 4 * kq, f1, fi, f2);
+    oz_digits(q, sh_e[rl], r0 + rl, kq, c, tile + (size_t)rl * ldt + c * oz::KC + 4 * kq);
   }
 }
 
@@ -299,8 +322,6 @@ __global__ void __launch_bounds__(256, 3) ozaki_split_kernel(const OzSplitProble
   // store covers a 128-byte core matrix of one digit slice
   const int rl = warp * 8 + (lane >> 2);
   const int kq = lane & 3;
-  double f1, fi, f2;
-  oz_row_factors(sh_e[rl], q.conj, f1, fi, f2);
   // asynchronous staging of chunk c into buffer b (zero-filled outside Y)
   auto stage = [&](int c, int b) {
     const int kbase = c * oz::KC;
@@ -339,7 +360,7 @@ __global__ void __launch_bounds__(256, 3) ozaki_split_kernel(const OzSplitProble
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
     __syncthreads();
-    oz_store_digits(q, r0 + rl, kq, c, &tile[b][rl][4 * kq], f1, fi, f2);
+    oz_digits(q, sh_e[rl], r0 + rl, kq, c, &tile[b][rl][4 * kq]);
     __syncthreads();
   }
 }
@@ -998,12 +1019,10 @@ size_t ozaki_mma_smem_bytes() { return (size_t)oz::STAGES * oz::STAGE; }
 constexpr size_t kSplitSmem = 2 * oz::SPLIT_ROWS * 33 * sizeof(cplx);
 
 // single-read split: rows per CTA for a step whose largest k_pad is kp (0: two-pass kernel)
-constexpr int split1_rows(int kp) { return kp <= 128 ? 32 : kp <= 256 ? 16 : kp <= 512 ? 8 : 0; }
+constexpr int split1_rows(int kp) { return kp <= 128 ? 16 : kp <= 512 ? 8 : 0; }
 constexpr size_t split1_smem(int kp) { return (size_t)split1_rows(kp) * (kp + 1) * sizeof(cplx); }
-constexpr size_t kSplit1SmemMax = 32 * 129 * sizeof(cplx);  // the largest of the three cases (66,048 B)
-static_assert(split1_smem(128) <= kSplit1SmemMax && split1_smem(256) <= kSplit1SmemMax &&
-                  split1_smem(512) <= kSplit1SmemMax,
-              "single-read split staging");
+constexpr size_t kSplit1SmemMax = split1_smem(512);  // the largest case (65,664 B)
+static_assert(split1_smem(128) <= kSplit1SmemMax && split1_smem(256) <= kSplit1SmemMax, "single-read split staging");
 
 cudaError_t ozaki_prepare() {
   static PerDevice set;
@@ -1027,9 +1046,6 @@ cudaError_t ozaki_prepare() {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(ozaki_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSplitSmem);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(ozaki_split1_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kSplit1SmemMax);
-  if (e == cudaSuccess)
     e = cudaFuncSetAttribute(ozaki_split1_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kSplit1SmemMax);
   if (e == cudaSuccess)
@@ -1052,8 +1068,7 @@ cudaError_t launch_ozaki_split(const void* probs, int nprob, int max_rows_pad, i
   dim3 grid(max_rows_pad / R, nprob);
   const int ldt = max_k_pad + 1;
   const size_t smem = split1_smem(max_k_pad);
-  if (R == 32) ozaki_split1_kernel<32><<<grid, 256, smem, st>>>(p, ldt);
-  else if (R == 16) ozaki_split1_kernel<16><<<grid, 256, smem, st>>>(p, ldt);
+  if (R == 16) ozaki_split1_kernel<16><<<grid, 256, smem, st>>>(p, ldt);
   else ozaki_split1_kernel<8><<<grid, 256, smem, st>>>(p, ldt);
   return cudaGetLastError();
 }
