@@ -529,7 +529,7 @@ void Plan::getrf(const std::vector<LuSpec>& specs) {
     if (s.n <= 0) continue;
     ZLuProblem p;
     p.A = s.A; p.ipiv = s.ipiv; p.Linv = s.Linv; p.T = s.T; p.info = s.info;
-    p.n = s.n; p.ld = s.ld; p.nopiv = s.nopiv ? 1 : 0; p.pad_ = 0;
+    p.n = s.n; p.ld = s.ld;
     v.push_back(p);
     max_n = std::max(max_n, s.n);
   }
@@ -564,52 +564,142 @@ void Plan::getrf(const std::vector<LuSpec>& specs) {
   }
 }
 
-void Plan::trtri(const std::vector<TriSpec>& specs, bool upper) {
-  std::vector<ZTriProblem> v;
+// Scratch of the joins: the products of all pairs of a level, or of one block column.
+size_t tri_scratch(int n) { return (size_t)std::max(n, kTriJoin) * kTriJoin; }
+
+// With the diagonal blocks of 32 inverted, neighbouring blocks are joined to
+// blocks of kTriJoin (upper: X12 = -(X11 U12) X22, lower: X21 = -X22 (L21 X11)),
+// two launches per doubling over all pairs of all matrices; then block columns
+// (upper) and rows (lower) of that width follow one after the other, two
+// launches each.  Joining all the way up would take fewer launches, but
+// compounds the rounding of each level.
+void Plan::tri_join(const std::vector<TriSpec>& up, const std::vector<TriSpec>& lo) {
   int max_n = 0;
-  std::vector<ZBlockOp> zero;
-  for (const auto& s : specs) {
-    if (s.n <= 0) continue;
-    ZTriProblem p;
-    p.A = s.A; p.X = s.X; p.n = s.n; p.lda = s.lda; p.ldx = s.ldx; p.pad_ = 0;
-    v.push_back(p);
-    max_n = std::max(max_n, s.n);
-    ZBlockOp z{};
-    z.C = s.X; z.ldc = s.ldx; z.m = z.n = s.n; z.kind = ZOP_FILL;
-    zero.push_back(z);
-  }
-  if (v.empty()) return;
-  blockops(zero);
-  const int nb = kTriNb;
-  Step s;
-  s.kind = Step::TRI_DIAG;
-  s.off = push_bytes(v.data(), v.size() * sizeof(ZTriProblem));
-  s.count = (int)v.size(); s.nb = nb; s.blocked = upper ? 1 : 0; s.max_n = max_n;
-  s.smem = ztrtri_smem_bytes(nb);
-  steps.push_back(s);
-  const int q = (max_n + nb - 1) / nb;
-  for (int j = 1; j < q; ++j) {
-    std::vector<ZGemmProblem> g1, g2;
-    for (size_t t = 0; t < v.size(); ++t) {
-      const ZTriProblem& p = v[t];
-      const TriSpec& sp = specs[t];
-      int j0 = j * nb;
-      if (j0 >= p.n) continue;
-      int wj = std::min(nb, p.n - j0);
-      if (upper) {
-        // T = X[0:j0, 0:j0] U[0:j0, j-block];  X[0:j0, j-block] = -T X[j-block, j-block]
-        g1.push_back(gp(p.X, p.ldx, p.A + (size_t)j0 * p.lda, p.lda, sp.T, p.n, j0, wj, j0, ONE));
-        g2.push_back(gp(sp.T, p.n, p.X + j0 + (size_t)j0 * p.ldx, p.ldx, p.X + (size_t)j0 * p.ldx, p.ldx, j0, wj,
-                        wj, MONE));
-      } else {
-        // T = L[j-block, 0:j0] Y[0:j0, 0:j0];  Y[j-block, 0:j0] = -Y[j-block, j-block] T
-        g1.push_back(gp(p.A + j0, p.lda, p.X, p.ldx, sp.T, nb, wj, j0, j0, ONE));
-        g2.push_back(gp(p.X + j0 + (size_t)j0 * p.ldx, p.ldx, sp.T, nb, p.X + j0, p.ldx, wj, j0, wj, MONE));
-      }
+  for (const auto* v : {&up, &lo})
+    for (const auto& p : *v) max_n = std::max(max_n, p.n);
+  // one join: block rows / columns [j, j + s) and [k, k + s2), k = j + s
+  auto join = [&](const TriSpec& p, bool upper, int j, int s, int s2, cplx* T, std::vector<ZGemmProblem>& g1,
+                  std::vector<ZGemmProblem>& g2) {
+    const int k = j + s;
+    cplx* X11 = p.X + j + (size_t)j * p.ldx;
+    cplx* X22 = p.X + k + (size_t)k * p.ldx;
+    if (upper) {
+      g1.push_back(gp(X11, p.ldx, p.A + j + (size_t)k * p.lda, p.lda, T, s, s, s2, s, ONE));
+      g2.push_back(gp(T, s, X22, p.ldx, p.X + j + (size_t)k * p.ldx, p.ldx, s, s2, s2, MONE));
+    } else {
+      g1.push_back(gp(p.A + k + (size_t)j * p.lda, p.lda, X11, p.ldx, T, s2, s2, s, s, ONE));
+      g2.push_back(gp(X22, p.ldx, T, s2, p.X + k + (size_t)j * p.ldx, p.ldx, s2, s, s2, MONE));
     }
+  };
+  for (int s = kTriNb; s < std::min(max_n, kTriJoin); s *= 2) {
+    std::vector<ZGemmProblem> g1, g2;
+    for (const auto* v : {&up, &lo})
+      for (const auto& p : *v) {
+        size_t t = 0;
+        for (int j = 0; j + s < p.n; j += 2 * s) {
+          const int s2 = std::min(s, p.n - j - s);
+          join(p, v == &up, j, s, s2, p.T + t, g1, g2);
+          t += (size_t)s * s2;
+        }
+      }
     gemm_fp64('N', 'N', g1);
     gemm_fp64('N', 'N', g2);
   }
+  for (int s = kTriJoin; s < max_n; s += kTriJoin) {
+    std::vector<ZGemmProblem> g1, g2;
+    for (const auto* v : {&up, &lo})
+      for (const auto& p : *v)
+        if (s < p.n) join(p, v == &up, 0, s, std::min(kTriJoin, p.n - s), p.T, g1, g2);
+    gemm_fp64('N', 'N', g1);
+    gemm_fp64('N', 'N', g2);
+  }
+}
+
+void Plan::trtri(const std::vector<TriSpec>& up, const std::vector<TriSpec>& lo) {
+  std::vector<ZBlockOp> zero;
+  for (const auto* list : {&up, &lo})
+    for (const auto& s : *list) {
+      if (s.n <= 0) continue;
+      ZBlockOp z{};
+      z.C = s.X; z.ldc = s.ldx; z.m = z.n = s.n; z.kind = ZOP_FILL;
+      zero.push_back(z);
+    }
+  if (zero.empty()) return;
+  blockops(zero);
+  for (const auto* list : {&up, &lo}) {
+    std::vector<ZTriProblem> v;
+    int max_n = 0;
+    for (const auto& s : *list) {
+      if (s.n <= 0) continue;
+      ZTriProblem p;
+      p.A = s.A; p.X = s.X; p.n = s.n; p.lda = s.lda; p.ldx = s.ldx; p.pad_ = 0;
+      v.push_back(p);
+      max_n = std::max(max_n, s.n);
+    }
+    if (v.empty()) continue;
+    Step s;
+    s.kind = Step::TRI_DIAG;
+    s.off = push_bytes(v.data(), v.size() * sizeof(ZTriProblem));
+    s.count = (int)v.size(); s.nb = kTriNb; s.blocked = list == &up ? 1 : 0; s.max_n = max_n;
+    s.smem = ztrtri_smem_bytes(kTriNb);
+    steps.push_back(s);
+  }
+  tri_join(up, lo);
+}
+
+// Unpivoted LU in panels of 32, three launches each: the diagonal block with the
+// inverses of its factors, F21 = A21 U^{-1} and F12 = L^{-1} A12 by substitution,
+// A22 -= F21 F12; then the joins of the triangular inverses.  A 512 block with its
+// inverses: 62 launches, 1.2 ms for 8 systems (panels of 16 whole columns, row
+// swaps and inverses in columns of 32: 190 launches, 3.7 ms); bound by the latency
+// of the launches' serial substitutions.
+void Plan::lu_nopiv(const std::vector<LuInvSpec>& specs) {
+  constexpr int nb = kTriNb;
+  std::vector<ZLuDiagProblem> v;
+  std::vector<ZBlockOp> zero, back;
+  std::vector<TriSpec> up, lo;
+  int max_n = 0;
+  for (const auto& s : specs) {
+    ZLuDiagProblem p;
+    p.A = s.A; p.F = s.F; p.Xu = s.Xu; p.Xl = s.Xl; p.info = s.info;
+    p.n = s.n; p.ld = s.ld; p.ldf = s.n; p.pad_ = 0;
+    v.push_back(p);
+    max_n = std::max(max_n, s.n);
+    for (cplx* X : {s.Xu, s.Xl}) {
+      ZBlockOp z{};
+      z.C = X; z.ldc = z.m = z.n = s.n; z.kind = ZOP_FILL;
+      zero.push_back(z);
+    }
+    ZBlockOp c{};
+    c.A = s.F; c.lda = s.n; c.C = s.A; c.ldc = s.ld; c.m = c.n = s.n; c.kind = ZOP_COPY;
+    back.push_back(c);
+    up.push_back({s.F, s.n, s.n, s.Xu, s.n, s.T});
+    lo.push_back({s.F, s.n, s.n, s.Xl, s.n, s.T + tri_scratch(s.n)});
+  }
+  if (v.empty()) return;
+  blockops(zero);
+  const size_t off = push_bytes(v.data(), v.size() * sizeof(ZLuDiagProblem));
+  for (int k0 = 0; k0 < max_n; k0 += nb) {
+    Step d;
+    d.kind = Step::LU_PANEL;
+    d.off = off; d.count = (int)v.size(); d.k0 = k0; d.nb = 0;
+    steps.push_back(d);
+    if (max_n <= k0 + nb) break;
+    d.nb = -1;
+    d.max_n = max_n;
+    steps.push_back(d);
+    std::vector<ZGemmProblem> g;
+    for (const auto& s : specs) {
+      const int k1 = k0 + nb, rest = s.n - k1;
+      if (rest <= 0) continue;
+      cplx* A22 = s.A + k1 + (size_t)k1 * s.ld;
+      g.push_back(gp(s.F + k1 + (size_t)k0 * s.n, s.n, s.F + k0 + (size_t)k1 * s.n, s.n, A22, s.ld, rest, rest, nb,
+                     MONE, A22, s.ld, ONE));
+    }
+    gemm_fp64('N', 'N', g);
+  }
+  blockops(back);
+  tri_join(up, lo);
 }
 
 void Plan::blockops(const std::vector<ZBlockOp>& ops) {
@@ -794,6 +884,11 @@ cudaError_t Plan::launch_step(const Step& s, const unsigned char* base, cudaStre
         e = launch_ztrace_prod(base + s.off, s.count, stream);
         break;
       case Step::LU_PANEL:
+        if (s.nb <= 0) {
+          e = s.nb == 0 ? launch_zlu_diag(base + s.off, s.count, s.k0, stream)
+                        : launch_zlu_solve(base + s.off, s.count, s.k0, s.max_n, stream);
+          break;
+        }
         e = launch_zgetrf_panel(base + s.off, s.count, s.k0, s.nb, s.smem, stream);
         break;
       case Step::LU_SWAP:

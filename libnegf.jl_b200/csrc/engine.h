@@ -47,6 +47,10 @@ size_t ztrtri_smem_bytes(int nb);
 cudaError_t zlu_prepare(size_t panel_smem, size_t tri_smem);
 cudaError_t launch_zgetrf_panel(const void* probs, int nprob, int k0, int nb, size_t smem, cudaStream_t st);
 cudaError_t launch_zlaswp_copy(const void* probs, int nprob, int k0, int nb, int max_n, cudaStream_t st);
+// unpivoted LU in panels of 32 (LU_PANEL steps): diagonal block (nb = 0), then the
+// rows below and the columns right of it (nb = -1)
+cudaError_t launch_zlu_diag(const void* probs, int nprob, int k0, cudaStream_t st);
+cudaError_t launch_zlu_solve(const void* probs, int nprob, int k0, int max_n, cudaStream_t st);
 cudaError_t launch_ztrtri_diag(const void* probs, int nprob, int nb, int upper, int max_n, size_t smem,
                                cudaStream_t st);
 
@@ -90,10 +94,18 @@ struct LuSpec {
   cplx* Linv;  // scratch nb x nb
   cplx* T;     // scratch nb x n
   int* info;
-  bool nopiv = false;  // lu(A, NoPivot()): no row interchanges
+};
+// Unpivoted LU (lu(A, NoPivot())) with both triangular inverses: A receives the
+// packed factors, Xu / Xl the inverses; F is scratch n x n.
+struct LuInvSpec {
+  cplx* A;
+  int n, ld;
+  cplx *Xu, *Xl, *F;
+  cplx* T;  // scratch tri_scratch(n) each for Xu and Xl
+  int* info;
 };
 // Triangular inverse request: X = inverse of the upper (non-unit) or unit
-// lower triangle of the packed factors A; T is scratch n x nb.
+// lower triangle of the packed factors A; T is scratch of tri_scratch(n).
 struct TriSpec {
   const cplx* A;
   int n, lda;
@@ -101,7 +113,8 @@ struct TriSpec {
   int ldx;
   cplx* T;
 };
-constexpr int kTriNb = 32;
+constexpr int kTriNb = 32, kTriJoin = 64;
+size_t tri_scratch(int n);
 int lu_panel_width(int max_n);
 
 struct ZTraceProblemHost {
@@ -193,7 +206,10 @@ class Plan {
   void blockops(const std::vector<ZBlockOp>& ops);
   void trace(const std::vector<ZTraceProblemHost>& probs);
   void getrf(const std::vector<LuSpec>& specs);
-  void trtri(const std::vector<TriSpec>& specs, bool upper);
+  // unpivoted LU and the inverses of both factors
+  void lu_nopiv(const std::vector<LuInvSpec>& specs);
+  // inverses of upper and of unit lower triangles, in the same launches
+  void trtri(const std::vector<TriSpec>& up, const std::vector<TriSpec>& lo);
 
   // Uploads the descriptors, zeroes the workspace and sets kernel attributes:
   // in order on `stream` (run calls it), or, without one, complete on return.
@@ -225,6 +241,7 @@ class Plan {
 
  private:
   cudaError_t launch_step(const Step& s, const unsigned char* base, cudaStream_t stream);
+  void tri_join(const std::vector<TriSpec>& up, const std::vector<TriSpec>& lo);
   size_t push_bytes(const void* p, size_t n);
   void* raw_alloc(size_t bytes);
   void* take_chunk(size_t bytes);

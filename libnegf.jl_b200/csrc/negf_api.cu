@@ -1211,7 +1211,7 @@ size_t selinv_bytes_per_energy(const negf_device_s& d, int method, int d1, bool 
     c += 10 * sd;                                           // Schur complement and 12 / 21 / 11 temporaries
     ops = 6;
   } else {
-    c += 2 * sd + (2 * n + 2) * mb * mb + 64 * mb * n;      // factor inverses, scratch, LU / trtri scratch
+    c += 2 * sd + (2 * n + 4) * mb * mb;                    // factor inverses, scratch, LU / triangular scratch
   }
   size_t bytes = c * sizeof(cplx) + 64 * n;
   if (mixed) {

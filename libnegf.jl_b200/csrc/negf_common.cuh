@@ -49,6 +49,33 @@ __host__ __device__ inline cplx cinv(cplx a) {
     return make_double2(r / d, -1.0 / d);
   }
 }
+#ifdef __CUDACC__
+// 1/a (0 for a = 0, and for infinite a).  a is scaled by a power of two
+// (exact), so that d = |a|^2 lies within [2^-102, 32); 1/d starts from a
+// single-precision reciprocal and takes one third-order Newton-Raphson step,
+// x (1 + e + e^2) with e = 1 - d x: |e| < 2^-21, so the step's error e^3 is
+// below the FP64 rounding.  No branch and no compare on the FP64 pipe: its
+// latency is part of every column's.
+__device__ __forceinline__ cplx cinv_pivot(cplx a) {
+  const int hx = __double2hiint(a.x) & 0x7fffffff, hy = __double2hiint(a.y) & 0x7fffffff;
+  const int e = max(hx, hy) >> 20;
+  const double s = __hiloint2double(max(1, 2046 - e) << 20, 0);
+  const double x = a.x * s, y = a.y * s;
+  const double d = fma(x, x, y * y);
+  float xf;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(xf) : "f"((float)d));
+  const double x0 = xf;
+  const double r = fma(-d, x0, 1.0);
+  const double t = fma(x0, fma(r, r, r), x0);
+  const bool none = (hx | hy | __double2loint(a.x) | __double2loint(a.y)) == 0 || e == 0x7ff;
+  return none ? make_double2(0.0, 0.0) : make_double2(x * t * s, -y * t * s);
+}
+
+// a - b c with four fused operations
+__device__ __forceinline__ cplx cfms_fused(cplx a, cplx b, cplx c) {
+  return make_double2(fma(b.y, c.y, fma(-b.x, c.x, a.x)), fma(-b.y, c.x, fma(-b.x, c.y, a.y)));
+}
+#endif
 // |re| + |im|: the pivot magnitude LAPACK's izamax uses (dcabs1)
 __host__ __device__ inline double cabs1(cplx a) { return fabs(a.x) + fabs(a.y); }
 
@@ -92,8 +119,6 @@ struct ZLuProblem {
   cplx* T;       // scratch nb x n (A12 copy)
   int* info;
   int n, ld;
-  int nopiv;     // 1: no row interchanges (the pivot of column c is row c)
-  int pad_;
 };
 
 // One matrix of a batched triangular inverse (zlu.cu).
@@ -101,6 +126,17 @@ struct ZTriProblem {
   const cplx* A;  // packed factors, n x n, lda
   cplx* X;        // output, n x n, ldx
   int n, lda, ldx, pad_;
+};
+
+// One matrix of a batched unpivoted LU with the inverses of its diagonal blocks
+// (zlu.cu): F receives the packed factors of the blocks, Xu / Xl (n x n, ld n)
+// the inverses of their upper and unit lower triangles.
+struct ZLuDiagProblem {
+  const cplx* A;
+  cplx* F;
+  cplx *Xu, *Xl;
+  int* info;
+  int n, ld, ldf, pad_;
 };
 
 // Digit split of one real-and-imaginary operand view for the Ozaki GEMM

@@ -70,7 +70,7 @@ int run_sync(Plan& plan, cudaStream_t st, int* dinfo, int n, const char* what) {
 }
 
 // LU request of one block with plan-owned scratch.
-LuSpec lu_spec(Plan& plan, cplx* A, int n, int ld, int* info, bool nopiv) {
+LuSpec lu_spec(Plan& plan, cplx* A, int n, int ld, int* info) {
   const int nb = lu_panel_width(n);
   LuSpec s;
   s.A = A; s.n = n; s.ld = ld;
@@ -78,14 +78,13 @@ LuSpec lu_spec(Plan& plan, cplx* A, int n, int ld, int* info, bool nopiv) {
   s.Linv = plan.alloc_c((size_t)nb * nb);
   s.T = plan.alloc_c((size_t)nb * n);
   s.info = info;
-  s.nopiv = nopiv;
   return s;
 }
 
 TriSpec tri_spec(Plan& plan, const cplx* A, int n, int lda, cplx* X) {
   TriSpec t;
   t.A = A; t.n = n; t.lda = lda; t.X = X; t.ldx = n;
-  t.T = plan.alloc_c((size_t)n * kTriNb);
+  t.T = plan.alloc_c(tri_scratch(n));
   return t;
 }
 
@@ -115,14 +114,19 @@ int build_selected_inverse(Plan& plan, std::vector<SelInvSystem>& S, int npl, in
     tmp[s] = plan.alloc_c(bb * (size_t)std::max(2 * npl + 2, 10));
   }
   auto scratch = [&](int s, int k) { return tmp[s] + bb * k; };
+  // scratch of the triangular inverses and of the LU, used by one step at a time
+  std::vector<cplx*> triT(ns), F(ns);
+  for (int s = 0; s < ns; ++s) {
+    triT[s] = plan.alloc_c(2 * tri_scratch(b));
+    if (nopiv) F[s] = plan.alloc_c(bb);
+  }
   auto inverses = [&](int i) {
     std::vector<TriSpec> up, lo;
     for (int s = 0; s < ns; ++s) {
-      up.push_back(tri_spec(plan, at(s, i, i), b, b, Uinv[s][i]));
-      lo.push_back(tri_spec(plan, at(s, i, i), b, b, Linv[s][i]));
+      up.push_back({at(s, i, i), b, b, Uinv[s][i], b, triT[s]});
+      lo.push_back({at(s, i, i), b, b, Linv[s][i], b, triT[s] + tri_scratch(b)});
     }
-    plan.trtri(up, true);
-    plan.trtri(lo, false);
+    plan.trtri(up, lo);
   };
   if (mode & 1) {
     // Block_factorization! (selected_inverse.jl:9-55).  Fill-in blocks are
@@ -132,10 +136,17 @@ int build_selected_inverse(Plan& plan, std::vector<SelInvSystem>& S, int npl, in
     for (int i = 0; i < npl; ++i) {
       // :18, be_getrf! (backend_cpu.jl:255-265: LAPACK getrf whose pivots the
       // reference discards) or lu(NoPivot()), the factorisation :17 names
-      std::vector<LuSpec> lus;
-      for (int s = 0; s < ns; ++s) lus.push_back(lu_spec(plan, at(s, i, i), b, b, S[s].info + i, nopiv));
-      plan.getrf(lus);
-      inverses(i);
+      if (nopiv) {
+        std::vector<LuInvSpec> lus;
+        for (int s = 0; s < ns; ++s)
+          lus.push_back({at(s, i, i), b, b, Uinv[s][i], Linv[s][i], F[s], triT[s], S[s].info + i});
+        plan.lu_nopiv(lus);
+      } else {
+        std::vector<LuSpec> lus;
+        for (int s = 0; s < ns; ++s) lus.push_back(lu_spec(plan, at(s, i, i), b, b, S[s].info + i));
+        plan.getrf(lus);
+        inverses(i);
+      }
       std::vector<ZBlockOp> cp;
       std::vector<ZGemmProblem> g;
       for (int s = 0; s < ns; ++s) {
@@ -339,7 +350,7 @@ int negf_ztrsm_batched(char side, char uplo, char trans, char diag, const double
       else
         g.push_back(gp(Bc, m[i], X, t, static_cast<cplx*>(B[i]), ldb[i], m[i], n[i], t, al));
     }
-    plan.trtri(tri, uplo == 'U');
+    plan.trtri(uplo == 'U' ? tri : std::vector<TriSpec>(), uplo == 'U' ? std::vector<TriSpec>() : tri);
     plan.blockops(cp);
     plan.gemm('N', 'N', g);
     return run_sync(plan, static_cast<cudaStream_t>(stream), nullptr, 0, "negf_ztrsm_batched");
@@ -363,8 +374,7 @@ int negf_zgetri_nopiv_batched(int32_t nprob, const int32_t* n, void* const* A, c
       lo.push_back(tri_spec(plan, static_cast<const cplx*>(A[i]), n[i], lda[i], Y));
       g.push_back(gp(X, n[i], Y, n[i], static_cast<cplx*>(A[i]), lda[i], n[i], n[i], n[i], ONE));
     }
-    plan.trtri(up, true);
-    plan.trtri(lo, false);
+    plan.trtri(up, lo);
     plan.gemm('N', 'N', g);
     return run_sync(plan, static_cast<cudaStream_t>(stream), nullptr, 0, "negf_zgetri_nopiv_batched");
   } catch (const std::bad_alloc&) {

@@ -32,32 +32,6 @@ struct GjPanelArgs {
   int blocked; // 0: whole matrix in one panel; 1: zgj_update_kernel follows; 2: write F and Bbuf for a GEMM update
 };
 
-// 1/a (0 for a = 0, and for infinite a).  a is scaled by a power of two
-// (exact), so that d = |a|^2 lies within [2^-102, 32); 1/d starts from a
-// single-precision reciprocal and takes one third-order Newton-Raphson step,
-// x (1 + e + e^2) with e = 1 - d x: |e| < 2^-21, so the step's error e^3 is
-// below the FP64 rounding.  No branch and no compare on the FP64 pipe: its
-// latency is part of every column's.
-__device__ __forceinline__ cplx gj_pivot_inv(cplx a) {
-  const int hx = __double2hiint(a.x) & 0x7fffffff, hy = __double2hiint(a.y) & 0x7fffffff;
-  const int e = max(hx, hy) >> 20;
-  const double s = __hiloint2double(max(1, 2046 - e) << 20, 0);
-  const double x = a.x * s, y = a.y * s;
-  const double d = fma(x, x, y * y);
-  float xf;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(xf) : "f"((float)d));
-  const double x0 = xf;
-  const double r = fma(-d, x0, 1.0);
-  const double t = fma(x0, fma(r, r, r), x0);
-  const bool none = (hx | hy | __double2loint(a.x) | __double2loint(a.y)) == 0 || e == 0x7ff;
-  return none ? make_double2(0.0, 0.0) : make_double2(x * t * s, -y * t * s);
-}
-
-// a - b c with four fused operations
-__device__ __forceinline__ cplx gj_cfms(cplx a, cplx b, cplx c) {
-  return make_double2(fma(b.y, c.y, fma(-b.x, c.x, a.x)), fma(-b.y, c.x, fma(-b.x, c.y, a.y)));
-}
-
 __device__ __forceinline__ void gj_cp16(cplx* smem, const cplx* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem));
 }
@@ -186,7 +160,7 @@ __global__ void __launch_bounds__(T, 1)
           if (RT == 1 || tid + k * T == 1023 - (int)(key & 1023u))
 #pragma unroll
             for (int q = 1; q < SW; ++q) ws[q] = a[k][q];
-        ws[0] = gj_pivot_inv(cand);
+        ws[0] = cinv_pivot(cand);
       }
       unsigned best = wkey;
       if (pw == 1) {
@@ -235,7 +209,7 @@ __global__ void __launch_bounds__(T, 1)
         const cplx x = row[q];
 #pragma unroll
         for (int k = 0; k < RT; ++k)
-          a[k][q - 1] = gj_cfms(prow[k] ? make_double2(0.0, 0.0) : a[k][q], f[k], x);
+          a[k][q - 1] = cfms_fused(prow[k] ? make_double2(0.0, 0.0) : a[k][q], f[k], x);
         if (q == 1) search();
       }
 #pragma unroll

@@ -15,8 +15,11 @@
 //   swap kernel: applies the panel's row interchanges to all other columns
 //     (LAPACK's zlaswp on both sides) and copies A12 into scratch;
 //   GEMMs (engine): A12 = L11^{-1} A12,  A22 -= A21 A12.
-// Triangular inverse (blocked by nb): diagonal blocks inverted in shared
-// memory here, off-diagonal blocks by GEMM recurrences in the engine.
+// Without row interchanges (the selected inverse of NEGF matrices) no panel of
+// whole columns is needed: a kernel factors a 32 x 32 diagonal block and inverts
+// its triangles, a second one substitutes A21 U^{-1} and L^{-1} A12, and the
+// engine forms the Schur update as a product.  Triangular inverse: diagonal blocks of 32 inverted in shared
+// memory here, then pairs of blocks joined by products, doubling their size.
 #include "negf_common.cuh"
 
 namespace negf {
@@ -42,13 +45,6 @@ __global__ void __launch_bounds__(LU_THREADS)
   }
   __syncthreads();
   for (int c = 0; c < w; ++c) {
-    if (p.nopiv) {  // block-uniform branch: lu(A, NoPivot())
-      if (tid == 0) {
-        *sp = c;
-        if (cabs1(S[(size_t)c * h + c]) <= 0.0 && p.info) atomicCAS(p.info, 0, k0 + c + 1);
-      }
-      __syncthreads();
-    } else {
     double bv = -1.0;
     int br = -1;
     for (int r = c + tid; r < h; r += LU_THREADS) {
@@ -79,7 +75,6 @@ __global__ void __launch_bounds__(LU_THREADS)
       }
     }
     __syncthreads();
-    }
     const int pr = *sp;
     if (tid == 0) p.ipiv[k0 + c] = k0 + pr;
     if (pr != c)
@@ -192,6 +187,138 @@ __global__ void ztrtri_diag_kernel(const ZTriProblem* __restrict__ probs, int nb
     int c = idx / w, r = idx - c * w;
     p.X[(j0 + r) + (size_t)(j0 + c) * p.ldx] = X[idx];
   }
+}
+
+// Unpivoted LU of the diagonal block [k0, k0 + w), w <= 32, and the inverses of
+// both factors, in shared memory: thread (row = lane, columns = warp + 8 q).
+// Step c takes l = S[:, c] / S[c, c] off the rows below -- of the block and of
+// the growing L^{-1} -- and needs one barrier, since it writes neither row nor
+// column c; the columns of L are divided at the end.  U^{-1} grows the same way
+// from the last column up.
+constexpr int kLuDiag = 32;
+__global__ void __launch_bounds__(256)
+    zlu_diag_kernel(const ZLuDiagProblem* __restrict__ probs, int k0) {
+  const ZLuDiagProblem p = probs[blockIdx.x];
+  if (k0 >= p.n) return;
+  constexpr int LD = kLuDiag + 1;
+  const int w = min(kLuDiag, p.n - k0), r = threadIdx.x & 31, j0 = threadIdx.x >> 5;
+  // Y: L^{-1} below the diagonal, U^{-1} (rows not yet divided) above, ones on it
+  constexpr int YO = kLuDiag * LD;
+  __shared__ cplx S[2 * YO], inv[kLuDiag];
+  cplx* const Y = S + YO;
+#pragma unroll
+  for (int j = j0; j < kLuDiag; j += 8) {
+    const cplx one = make_double2(r == j ? 1.0 : 0.0, 0.0);
+    S[j * LD + r] = r < w && j < w ? p.A[(k0 + r) + (size_t)(k0 + j) * p.ld] : one;
+    Y[j * LD + r] = one;
+  }
+  __syncthreads();
+  for (int c = 0; c < w; ++c) {
+    const cplx piv = S[c * LD + c];
+    const bool zero = piv.x == 0.0 && piv.y == 0.0;
+    const cplx iv = cinv_pivot(piv);
+    if (threadIdx.x == 0) {
+      inv[c] = iv;
+      if (zero && p.info) atomicCAS(p.info, 0, k0 + c + 1);
+    }
+    if (r > c) {
+      const cplx l = cmul(S[c * LD + r], iv);
+#pragma unroll
+      for (int j = j0; j < kLuDiag; j += 8) {
+        const int m = j * LD + (j > c ? 0 : YO);
+        S[m + r] = cfms_fused(S[m + r], l, S[m + c]);
+      }
+    }
+    __syncthreads();
+  }
+  for (int c = w - 1; c > 0; --c) {
+    if (r < c) {
+      const cplx u = cmul(S[c * LD + r], inv[c]);
+#pragma unroll
+      for (int j = j0; j < kLuDiag; j += 8)
+        if (j >= c) Y[j * LD + r] = cfms_fused(Y[j * LD + r], u, Y[j * LD + c]);
+    }
+    __syncthreads();
+  }
+  if (r < w)
+    for (int j = j0; j < w; j += 8) {
+      const size_t x = (size_t)(k0 + r) + (size_t)(k0 + j) * p.n;
+      p.F[(k0 + r) + (size_t)(k0 + j) * p.ldf] = r > j ? cmul(S[j * LD + r], inv[j]) : S[j * LD + r];
+      const cplx y = Y[j * LD + r], zero = make_double2(0.0, 0.0);
+      p.Xl[x] = r >= j ? y : zero;
+      p.Xu[x] = r <= j ? cmul(y, inv[r]) : zero;
+    }
+}
+
+// F21 = A21 U^{-1} and F12 = L^{-1} A12 of a panel by substitution, a thread per
+// row of A21 or column of A12.  (Products with the inverses of the diagonal block
+// would be faster, but without row interchanges U may have small pivots: the
+// selected inverse of NEGF matrices lost a digit.)
+__global__ void __launch_bounds__(64) zlu_solve_kernel(const ZLuDiagProblem* __restrict__ probs, int k0, int chunks) {
+  const ZLuDiagProblem p = probs[blockIdx.y];
+  const int k1 = k0 + kLuDiag;
+  const bool rows = (int)blockIdx.x < chunks;
+  const int i = k1 + (blockIdx.x - (rows ? 0 : chunks)) * 64 + threadIdx.x;
+  if (k1 + (int)(blockIdx.x - (rows ? 0 : chunks)) * 64 >= p.n) return;
+  __shared__ cplx T[kLuDiag * kLuDiag], d[kLuDiag];
+  for (int e = threadIdx.x; e < kLuDiag * kLuDiag; e += 64) {
+    const int r = e % kLuDiag, c = e / kLuDiag;  // T[row][column] of U, or of L transposed
+    T[rows ? r * kLuDiag + c : c * kLuDiag + r] = p.F[(k0 + r) + (size_t)(k0 + c) * p.ldf];
+  }
+  if (threadIdx.x < kLuDiag) {
+    const size_t q = k0 + threadIdx.x;
+    d[threadIdx.x] = p.Xu[q + q * p.n];
+  }
+  __syncthreads();
+  if (i >= p.n) return;
+  const cplx* src = rows ? p.A + i + (size_t)k0 * p.ld : p.A + k0 + (size_t)i * p.ld;
+  cplx* dst = rows ? p.F + i + (size_t)k0 * p.ldf : p.F + k0 + (size_t)i * p.ldf;
+  const size_t ss = rows ? p.ld : 1, ds = rows ? p.ldf : 1;
+  // right-looking substitution; the current column is always x[0] (or y[0]), so
+  // that the loops are not unrolled: the straight-line form was bound by its
+  // instruction fetches (22 us).  The slots past the last column hold leftovers.
+  cplx x[16], y[16];
+#pragma unroll
+  for (int c = 0; c < 16; ++c) {
+    x[c] = src[c * ss];
+    y[c] = src[(c + 16) * ss];
+  }
+#pragma unroll 1
+  for (int c = 0; c < 16; ++c) {
+    const cplx v = rows ? cmul(x[0], d[c]) : x[0];
+    const cplx* t = T + c * kLuDiag;
+    dst[c * ds] = v;
+#pragma unroll
+    for (int j = 1; j < 16; ++j) x[j - 1] = cfms_fused(x[j], v, t[min(c + j, 15)]);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) y[j] = cfms_fused(y[j], v, t[16 + j]);
+  }
+#pragma unroll 1
+  for (int c = 16; c < 32; ++c) {
+    const cplx v = rows ? cmul(y[0], d[c]) : y[0];
+    const cplx* t = T + c * kLuDiag;
+    dst[c * ds] = v;
+#pragma unroll
+    for (int j = 1; j < 16; ++j) y[j - 1] = cfms_fused(y[j], v, t[min(c + j, 31)]);
+  }
+}
+
+// max_n: the largest matrix; the panel at k0 is complete (k0 + 32 <= n) wherever rows follow it
+cudaError_t launch_zlu_solve(const void* probs, int nprob, int k0, int max_n, cudaStream_t st) {
+  const int rest = max_n - k0 - kLuDiag;
+  if (nprob <= 0 || rest <= 0) return cudaSuccess;
+  const int chunks = (rest + 63) / 64;
+  for (int base = 0; base < nprob; base += 65535) {  // grid.y is limited to 65535
+    const int cnt = nprob - base < 65535 ? nprob - base : 65535;
+    zlu_solve_kernel<<<dim3(2 * chunks, cnt), 64, 0, st>>>(static_cast<const ZLuDiagProblem*>(probs) + base, k0, chunks);
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_zlu_diag(const void* probs, int nprob, int k0, cudaStream_t st) {
+  if (nprob <= 0) return cudaSuccess;
+  zlu_diag_kernel<<<nprob, 256, 0, st>>>(static_cast<const ZLuDiagProblem*>(probs), k0);
+  return cudaGetLastError();
 }
 
 size_t zgetrf_panel_smem_bytes(int n, int nb) {
