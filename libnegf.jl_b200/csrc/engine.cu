@@ -1308,6 +1308,8 @@ void build_lead_pass(Plan& plan, const std::vector<TriSystem>& sys, std::vector<
       const auto& s = sys[k];
       if (i + 1 >= s.npl()) continue;
       v.push_back(gp(G[k][i], s.b[i], work[k].R[i], s.b[i], u[k], s.b[i], s.b[i], s.b[i + 1], s.b[i], MONE));
+      if (Q[k].t_out)  // beside the product with the same R_i: one digit split of it
+        v.push_back(gp(g0(k, i), s.b[0], work[k].R[i], s.b[i], g0(k, i + 1), s.b[0], s.b[0], s.b[i + 1], s.b[i], MONE));
     }
   };
   {
@@ -1326,8 +1328,6 @@ void build_lead_pass(Plan& plan, const std::vector<TriSystem>& sys, std::vector<
       const int b = s.b[i], b1 = s.b[i + 1];
       a.push_back(gp(w.L[i], b1, u[k], b, G[k][i + 1], b1, b1, b1, b, MONE, w.g[i + 1], b1, ONE));
       a.push_back(gp(u[k], b, t[k][i + 1], b1, ub[k], b, b, b1, b1, ONE));
-      if (Q[k].t_out)
-        a.push_back(gp(g0(k, i), s.b[0], w.R[i], b, g0(k, i + 1), s.b[0], s.b[0], b1, b, MONE));
       // gl[i] = i G^n_ii, so -G^n_ii / 2 is (i / 2) gl[i]
       c.push_back(gp(Q[k].gl[i], b, w.L[i], b1, ub[k], b, b, b1, b, make_double2(0.0, 0.5), ub[k], b, ONE));
       // t_{i+1} is done with: it takes n_{i+1} / 2 - L_{i+1} A
