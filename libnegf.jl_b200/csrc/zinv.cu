@@ -29,7 +29,7 @@ constexpr int SW = 8;  // columns of a sub-panel, factored in registers
 struct GjPanelArgs {
   int k0;      // first column of this panel
   int nb;      // panel width (columns)
-  int blocked; // 0: whole matrix in one panel; 1: zgj_update_kernel follows; 2: write F and Bbuf for a GEMM update
+  int blocked; // 1: zgj_update_kernel follows; 2: write F and Bbuf for a GEMM update
 };
 
 __device__ __forceinline__ void gj_cp16(cplx* smem, const cplx* gmem) {
@@ -76,8 +76,7 @@ __device__ __forceinline__ unsigned gj_key(double v, int row) {
 // one SM in the rank-8 updates.  Eight columns keep a row in 32 registers; wider
 // sub-panels do more of the n w^2 work in the latency-bound form, narrower ones
 // add update passes over shared memory.  A 256 x 32 panel takes 40 us (104 us
-// with the whole slab in registers and one rank-1 step per column), a whole 64 x
-// 64 inversion 57 us (192 us for 64 of them before), 100 x 100 117 us (627 us).
+// with the whole slab in registers and one rank-1 step per column).
 template <int T, int RT>
 __global__ void __launch_bounds__(T, 1)
     zgj_panel_kernel(const ZInvProblem* __restrict__ probs, GjPanelArgs args) {
@@ -304,17 +303,6 @@ __global__ void __launch_bounds__(T, 1)
   }
   __syncthreads();
 
-  if (!args.blocked) {
-    // whole matrix in one panel: write the un-permuted inverse directly,
-    // out[r, piv[c]] = S[piv[r], c]
-    if (dead) return;  // singular: info is set, out is left untouched
-    for (int c = warp; c < n; c += NW) {
-      cplx* o = p.out + (size_t)sh_piv[c] * p.ldo;
-      const cplx* Sc = S + (size_t)c * ldw;
-      for (int r = lane; r < n; r += 32) o[r] = Sc[sh_piv[r]];
-    }
-    return;
-  }
   // write back slab, pivots and used flags
   for (int j = warp; j < w; j += NW)
     for (int r = lane; r < n; r += 32) p.W[r + (size_t)(k0 + j) * p.ld] = S[(size_t)j * ldw + r];
@@ -345,6 +333,200 @@ __global__ void __launch_bounds__(T, 1)
   for (int e = tid; e < w * n; e += T) {
     const int j = e / w;
     p.Bbuf[e] = j < k0 || j >= k0 + w ? S[e] : make_double2(0.0, 0.0);
+  }
+}
+
+// The whole inversion of a matrix that fits shared memory (n <= 112): the same
+// sub-panels, with the next one factored beside the rank-8 updates by the
+// current one, once all warps have updated its 8 columns.  1, 2 or 4 warps factor
+// (n <= 32, 64, 112; one row per thread).  One or two are alone on their
+// scheduler partitions (warp mod 4): FP64 tensor instructions of a warp beside
+// them would delay every step of the column loop.  Odd CTAs take the opposite
+// partitions, so that CTAs that share an SM spread over all of them.
+// Bound: the latency of the column loop (750 to 1000 cycles a column) up to n =
+// 64, the FP64 pipes of one SM above.  Against one sub-panel and one update after
+// the other: one matrix of 50: 33 us (42), of 64: 38 (52), 592 of them 110 (124);
+// 512 of 32: 25 (41); one of 100: 108 (111), 296 of them 216 (224).  Two
+// factoring warps with two rows per thread take 7 % longer at 100.
+template <int T>
+__global__ void __launch_bounds__(T, 512 / T) zgj_whole_kernel(const ZInvProblem* __restrict__ probs) {
+  using gj::SW;
+  const ZInvProblem p = probs[blockIdx.x];
+  const int n = p.n;
+  if (n <= 0) return;
+  constexpr int NW = T / 32;
+  const int ldw = n | 1, wt = (n + SW - 1) / SW, mt = (n + 15) / 16;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx* S = reinterpret_cast<cplx*>(smem_raw);       // ldw x 8 wt
+  cplx* Bb = S + (size_t)ldw * SW * wt;               // 8 wt columns of 8 pivot-row values
+  cplx* slot = Bb + (size_t)SW * SW * wt;             // [2][4][SW] candidate rows
+  unsigned* part = reinterpret_cast<unsigned*>(slot + 8 * SW);  // [2][4] candidate keys
+  int* sh_piv = reinterpret_cast<int*>(part + 8);     // n
+  int* sh_dead = sh_piv + n;
+  uint8_t* at = reinterpret_cast<uint8_t*>(sh_dead + 1);  // n: the sub-panel whose pivot row a row is
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq = lane & 3;
+  const int pw = n > 64 ? 4 : n > 32 ? 2 : 1, PT = 32 * pw;  // warps that factor
+  const int pbase = pw == 4 ? 0 : pw == 2 ? 2 * (blockIdx.x & 1) : blockIdx.x & 3;
+  const int pidx = warp - pbase;  // 0 .. pw - 1: factors
+  const bool factors = pidx >= 0 && pidx < pw;
+  // the updating warps: those of the other partitions, or the second four
+  const int part4 = warp & 3, upart = 4 - pw;
+  const bool updates = pw == 4 ? warp >= 4 : part4 < pbase || part4 >= pbase + pw;
+  const int nu = pw == 4 ? NW - 4 : upart * (NW / 4);
+  const int uidx = pw == 4 ? warp - 4 : (part4 < pbase ? part4 : part4 - pw) + upart * (warp >> 2);
+  const int ptid = pidx * 32 + lane;
+
+  for (int j = warp; j < n; j += NW)
+    for (int r = lane; r < n; r += 32) gj_cp16(S + (size_t)j * ldw + r, p.W + r + (size_t)j * p.ld);
+  for (int r = tid; r < n; r += T) at[r] = 255;
+  if (tid == 0) *sh_dead = 0;
+  gj_cp_wait();
+  __syncthreads();
+
+  bool used = ptid >= n;
+
+  // Gauss-Jordan steps of columns [s0, s0 + 8), in registers (warps that factor)
+  auto factor = [&](int s0) {
+    const int sw = min(SW, n - s0);
+    cplx a[SW];
+#pragma unroll
+    for (int j = 0; j < SW; ++j)
+      a[j] = (ptid < n && j < sw) ? S[(size_t)(s0 + j) * ldw + ptid] : make_double2(0.0, 0.0);
+    unsigned key = 0, wkey = 0;
+    auto search = [&] {
+      const double v = cabs1(a[0]);
+      key = !used && __double2hiint(v) <= 0x7ff00000 ? gj_key(v, ptid) : 0u;
+      wkey = __reduce_max_sync(0xffffffffu, key);
+    };
+    search();
+#pragma unroll 1
+    for (int j = 0; j < sw; ++j) {
+      const int buf = (j & 1) * 4;
+      if (key == wkey && key != 0u) {
+        cplx* ws = slot + (buf + pidx) * SW;
+#pragma unroll
+        for (int q = 1; q < SW; ++q) ws[q] = a[q];
+        ws[0] = cinv_pivot(a[0]);
+      }
+      unsigned best = wkey;
+      if (pw == 1) {
+        __syncwarp();
+      } else {
+        if (lane == 0) part[buf + pidx] = wkey;
+        asm volatile("bar.sync 1, %0;" ::"r"(PT) : "memory");
+        best = max(part[buf], part[buf + 1]);
+        if (pw == 4) best = max(best, max(part[buf + 2], part[buf + 3]));
+      }
+      const int pr = 1023 - (int)(best & 1023u);
+      const cplx* row = slot + (buf + (pr % PT >> 5)) * SW;
+      if (best < 2048u) {  // no candidate row, or one whose leading bits are zero (uniform)
+        if (best == 0u) {
+          if (ptid == 0) {
+            *sh_dead = 1;
+            if (p.info) atomicCAS(p.info, 0, s0 + j + 1);
+          }
+          break;
+        }
+        if (ptid == 0 && p.info && row[0].x == 0.0 && row[0].y == 0.0) atomicCAS(p.info, 0, s0 + j + 1);
+      }
+      if (ptid == PT - 1) {
+        sh_piv[s0 + j] = pr;
+        at[pr] = (uint8_t)(s0 / SW);
+      }
+      const cplx pv = row[0];
+      const bool prow = ptid == pr;
+      const cplx f = prow ? cneg(pv) : cmul(a[0], pv);
+      used = used || prow;
+#pragma unroll
+      for (int q = 1; q < SW; ++q) {
+        // the product apart, as in the updates: 3 % less error, no time
+        const cplx x = row[q], c = prow ? make_double2(0.0, 0.0) : a[q];
+        a[q - 1] = make_double2(c.x + fma(f.y, x.y, -f.x * x.x), c.y - fma(f.y, x.x, f.x * x.y));
+        if (q == 1) search();
+      }
+      a[SW - 1] = cneg(f);
+    }
+#pragma unroll
+    for (int q = 0; q < SW; ++q) {
+      const int j = q - (SW - sw);
+      if (ptid < n && j >= 0) S[(size_t)(s0 + j) * ldw + ptid] = a[q];
+    }
+  };
+  // rank-8 update by sub-panel s of the column tiles [t0, t1) except s and skip, as
+  // worker w of nw: row tiles of 16, or with more workers than row tiles a share
+  // of the column tiles.  The products are summed apart and added to S last: in
+  // one chain on S the error of an inverse is 15 to 20 % larger (above n = 112 the
+  // rank-32 update sets the error, and the panels keep the one chain).
+  auto update = [&](int s, int t0, int t1, int skip, int w, int nw) {
+    const int sw = min(SW, n - s * SW), ms = min(mt, nw), ng = nw / ms;
+    if (w >= ms * ng) return;
+    const cplx z = make_double2(0.0, 0.0);
+    for (int m = w % ms; m < mt; m += ms) {
+      const int r0 = m * 16 + g, r1 = r0 + 8;
+      const bool i0 = r0 < n, i1 = r1 < n;
+      const bool o0 = i0 && at[r0] != s, o1 = i1 && at[r1] != s;  // pivot rows take the product alone
+      cplx x0[2], x1[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int kk = tq + 4 * h;
+        x0[h] = kk < sw && i0 ? S[(size_t)(s * SW + kk) * ldw + r0] : z;
+        x1[h] = kk < sw && i1 ? S[(size_t)(s * SW + kk) * ldw + r1] : z;
+      }
+      for (int ct = t0 + w / ms; ct < t1; ct += ng) {
+        if (ct == s || ct == skip) continue;
+        cplx* C0 = S + (size_t)(ct * SW + 2 * tq) * ldw + r0;
+        const cplx c00 = o0 ? C0[0] : z, c01 = o0 ? C0[ldw] : z, c10 = o1 ? C0[8] : z, c11 = o1 ? C0[ldw + 8] : z;
+        double rr[4] = {}, ri[4] = {}, ii[4] = {}, ir[4] = {};
+        const cplx* B = Bb + (size_t)(ct * SW + g) * SW;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const cplx y = B[(tq + 4 * h) ^ ((g & 1) << 2)];
+          gj_dmma(rr, x0[h].x, x1[h].x, y.x);
+          gj_dmma(ri, x0[h].x, x1[h].x, y.y);
+          gj_dmma(ii, x0[h].y, x1[h].y, y.y);
+          gj_dmma(ir, x0[h].y, x1[h].y, y.x);
+        }
+        if (i0) {
+          C0[0] = make_double2(c00.x + (rr[0] - ii[0]), c00.y + (ri[0] + ir[0]));
+          C0[ldw] = make_double2(c01.x + (rr[1] - ii[1]), c01.y + (ri[1] + ir[1]));
+        }
+        if (i1) {
+          C0[8] = make_double2(c10.x + (rr[2] - ii[2]), c10.y + (ri[2] + ir[2]));
+          C0[ldw + 8] = make_double2(c11.x + (rr[3] - ii[3]), c11.y + (ri[3] + ir[3]));
+        }
+      }
+    }
+  };
+
+  if (factors) factor(0);
+  __syncthreads();
+  for (int s = 0; s < wt; ++s) {
+    if (*sh_dead) return;  // singular: info is set, out is left untouched
+    if (wt == 1) break;
+    // the pivot rows in the other columns (unused k of a last, narrower tile: zero)
+    const int sw = min(SW, n - s * SW);
+    for (int i = tid; i < SW * SW * wt; i += T) {
+      const int q = i / SW, j = i % SW;
+      Bb[q * SW + (j ^ ((q & 1) << 2))] =
+          q < n && j < sw ? S[(size_t)q * ldw + sh_piv[s * SW + j]] : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    if (s + 1 == wt) {
+      update(s, 0, wt, -1, warp, NW);
+    } else {
+      update(s, s + 1, s + 2, -1, warp, NW);  // the next 8 columns first, by all warps
+      __syncthreads();
+      if (factors) factor((s + 1) * SW);
+      else if (updates) update(s, 0, wt, s + 1, uidx, nu);
+    }
+    __syncthreads();
+  }
+  // un-permuted: out[r, piv[c]] = S[piv[r], c]
+  for (int c = warp; c < n; c += NW) {
+    cplx* o = p.out + (size_t)sh_piv[c] * p.ldo;
+    const cplx* Sc = S + (size_t)c * ldw;
+    for (int r = lane; r < n; r += 32) o[r] = Sc[sh_piv[r]];
   }
 }
 
@@ -463,16 +645,17 @@ size_t zgj_panel_smem_bytes(int n, int nb) {
   return (b + 15) & ~size_t(15);
 }
 
-// One thread per row up to 256 rows, then two and four rows per thread.  Up to
-// 128 rows four warps, whose barriers are cheaper and whose CTAs share an SM --
-// except a whole matrix above 64, whose rank-8 updates want eight warps (n =
-// 100: 131 us against 162 us; n = 64: 62 against 58 us, 592 matrices 149 against
-// 130).
+// Panels: one thread per row up to 256 rows (four warps up to 128, whose barriers
+// are cheaper), then two and four rows per thread.  Whole matrices: four warps up
+// to 32 rows, then eight.
 cudaError_t launch_zgj_panel(const ZInvProblem* probs_dev, int nprob, int k0, int nb, int blocked, size_t smem,
                              cudaStream_t stream, int max_n) {
   if (nprob <= 0) return cudaSuccess;
   GjPanelArgs a{k0, nb, blocked};
-  if (max_n <= (blocked ? 128 : 64)) zgj_panel_kernel<128, 1><<<nprob, 128, smem, stream>>>(probs_dev, a);
+  if (!blocked) {
+    if (max_n <= 32) zgj_whole_kernel<128><<<nprob, 128, smem, stream>>>(probs_dev);
+    else zgj_whole_kernel<256><<<nprob, 256, smem, stream>>>(probs_dev);
+  } else if (max_n <= 128) zgj_panel_kernel<128, 1><<<nprob, 128, smem, stream>>>(probs_dev, a);
   else if (max_n <= 256) zgj_panel_kernel<256, 1><<<nprob, 256, smem, stream>>>(probs_dev, a);
   else if (max_n <= 512) zgj_panel_kernel<256, 2><<<nprob, 256, smem, stream>>>(probs_dev, a);
   else zgj_panel_kernel<256, 4><<<nprob, 256, smem, stream>>>(probs_dev, a);
@@ -509,6 +692,7 @@ cudaError_t zgj_prepare(size_t smem) {
   if (set.done(dev)) return cudaSuccess;
   for (const void* f : {(const void*)zgj_panel_kernel<128, 1>, (const void*)zgj_panel_kernel<256, 1>,
                         (const void*)zgj_panel_kernel<256, 2>, (const void*)zgj_panel_kernel<256, 4>,
+                        (const void*)zgj_whole_kernel<128>, (const void*)zgj_whole_kernel<256>,
                         (const void*)zgj_update_kernel<16>, (const void*)zgj_update_kernel<32>})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   if (e == cudaSuccess) set.set(dev);
