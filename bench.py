@@ -433,7 +433,7 @@ def run_ours(args):
             "algorithmic_tflops": step_flops / ((fms / args.steps) / 1000.0) / 1e12,
             "gpu_launches": int(fstats["launches"]) * args.steps,
             "kernels": breakdown_of(fprof),
-            "roofline": {"kernel": "zgemm3m_batched_kernel (DMMA m16n8k4 f64)", "bound": "tensor",
+            "roofline": {"kernel": "zgemm3m_tile_kernel (DMMA m16n8k4 f64)", "bound": "tensor",
                          "achieved": f_ach, "peak": fp64_peak, "unit": "TFLOP/s",
                          "frac": f_ach / fp64_peak if fp64_peak else None,
                          "peak_source": "FP64 mma.sync throughput measured in-run (negf_probe_fp64_peak)"}}
