@@ -831,10 +831,12 @@ cudaError_t Plan::run(cudaStream_t stream, bool use_graph) {
     if (e != cudaSuccess) return e;
   }
   const unsigned char* base = static_cast<const unsigned char*>(dblob_);
+  if (!use_graph) chain_ctas = 1 << 30;  // the first launch waits as usual
   for (const auto& s : steps) {
     e = launch_step(s, base, stream);
     if (e != cudaSuccess) break;
   }
+  chain_ctas = -1;
   if (use_graph) {
     cudaGraph_t g = nullptr;
     cudaError_t e2 = cudaStreamEndCapture(stream, &g);

@@ -71,6 +71,47 @@ __device__ __forceinline__ cplx cinv_pivot(cplx a) {
   return none ? make_double2(0.0, 0.0) : make_double2(x * t * s, -y * t * s);
 }
 
+// Chained launches.  A plan's kernels run one after the other on a stream; with
+// programmatic stream serialization the CTAs of the next kernel are placed as
+// soon as the current one's have started, instead of after its end and a
+// launch's latency (about 2 us: RGF of 10 layers of 32 487 -> 394 us).  Each
+// kernel calls chain_entry first: it lets the next one come, and waits until the
+// ones before have completed, so that everything after it sees what plain stream
+// order would show.  (Every kernel of a chain has to wait, also the CTAs that do
+// nothing: the next one's wait covers its predecessor alone.)
+__device__ __forceinline__ void chain_entry() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// CTAs of the kernel before in the calling thread's chain; negative outside one.
+// A chain is a plan's direct run: captured into a graph, the launches cost its
+// first pass more than they give (16 layers of 64, 64 energies: 2.7 -> 3.1 ms).
+// Two kernels are chained while together they have no more CTAs than the GPU has
+// SMs (148): above that the early CTAs share the SMs that are free first instead
+// of spreading over all of them (Keldysh sweep of 10 layers of 300: 7.4 ms plain,
+// 8.1 with every launch chained, 7.0 by this rule).
+inline thread_local long long chain_ctas = -1;
+
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = stream;
+  c.attrs = &attr;
+  const long long ctas = (long long)grid.x * grid.y * grid.z;
+  if (chain_ctas >= 0) {
+    c.numAttrs = chain_ctas + ctas <= 148 ? 1 : 0;
+    chain_ctas = ctas;
+  }
+  return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // a - b c with four fused operations
 __device__ __forceinline__ cplx cfms_fused(cplx a, cplx b, cplx c) {
   return make_double2(fma(b.y, c.y, fma(-b.x, c.x, a.x)), fma(-b.y, c.x, fma(-b.x, c.y, a.y)));

@@ -10,6 +10,7 @@ namespace negf {
 constexpr int EL_TILE = 32;
 
 __global__ void zblockop_kernel(const ZBlockOp* __restrict__ ops) {
+  chain_entry();
   ZBlockOp o = ops[blockIdx.z];
   if (o.alpha_ptr) o.alpha = *o.alpha_ptr;
   __shared__ cplx tile[EL_TILE][EL_TILE + 1];
@@ -83,7 +84,7 @@ cudaError_t launch_zblockops(const ZBlockOp* ops_dev, int nops, int max_m, int m
   for (int base = 0; base < nops; base += 65535) {
     int cnt = nops - base < 65535 ? nops - base : 65535;
     dim3 grid(tiles, 1, cnt);
-    zblockop_kernel<<<grid, dim3(EL_TILE, 8), 0, stream>>>(ops_dev + base);
+    launch_chained(zblockop_kernel, grid, dim3(EL_TILE, 8), 0, stream, ops_dev + base);
   }
   return cudaGetLastError();
 }
@@ -100,6 +101,7 @@ struct ZTraceProblem {
 };
 
 __global__ void ztrace_prod_kernel(const ZTraceProblem* __restrict__ probs) {
+  chain_entry();
   const ZTraceProblem p = probs[blockIdx.x];
   double sr = 0.0, si = 0.0;
   for (int idx = threadIdx.x; idx < p.n * p.n; idx += blockDim.x) {
@@ -131,7 +133,7 @@ __global__ void ztrace_prod_kernel(const ZTraceProblem* __restrict__ probs) {
 
 cudaError_t launch_ztrace_prod(const void* probs_dev, int nprob, cudaStream_t stream) {
   if (nprob <= 0) return cudaSuccess;
-  ztrace_prod_kernel<<<nprob, 256, 0, stream>>>(static_cast<const ZTraceProblem*>(probs_dev));
+  launch_chained(ztrace_prod_kernel, nprob, 256, 0, stream, static_cast<const ZTraceProblem*>(probs_dev));
   return cudaGetLastError();
 }
 

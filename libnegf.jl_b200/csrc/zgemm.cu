@@ -111,6 +111,7 @@ __device__ __forceinline__ void load_stage(cplx* As, cplx* Bs, const ZGemmProble
 template <bool TA, bool CA, bool TB, bool CB, bool PRE>
 __global__ void __launch_bounds__(gemm::THREADS, 2)
     zgemm_batched_kernel(const ZGemmProblem* __restrict__ probs, const int* __restrict__ tile_start, int nprob) {
+  chain_entry();
   using namespace gemm;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx* smem = reinterpret_cast<cplx*>(smem_raw);
@@ -267,6 +268,7 @@ constexpr size_t smem_bytes() {
 template <bool TA, bool CA, bool TB, bool CB, int WM, int WN, int WK>
 __global__ void __launch_bounds__(gemm_st::THREADS, 4)
     zgemm3m_tile_kernel(const ZGemmProblem* __restrict__ probs, const int* __restrict__ tile_start, int nprob) {
+  chain_entry();
   using namespace gemm_st;
   static_assert(WM * WN * WK * 32 == THREADS, "warp layout");
   static_assert(WK == 1 || (size_t)WM * WN * (WK - 1) * 24 * 32 * sizeof(double) <= smem_bytes<WM, WN>(), "partial sums");
@@ -507,15 +509,15 @@ cudaError_t launch_zgemm_batched_ex(char opA, char opB, bool preload, const ZGem
   if (form == kFormTile32 || form == kFormTile16) {
     const int ia = op_index(opA), ib = op_index(opB);
     if (form == kFormTile32)
-      pick_tile_t<2, 2, 1>(ia, ib)<<<total_tiles, gemm_st::THREADS, gemm_st::smem_bytes<2, 2>(), stream>>>(
-          probs_dev, tile_start_dev, nprob);
+      launch_chained(pick_tile_t<2, 2, 1>(ia, ib), total_tiles, gemm_st::THREADS, gemm_st::smem_bytes<2, 2>(), stream,
+                     probs_dev, tile_start_dev, nprob);
     else
-      pick_tile_t<1, 1, 4>(ia, ib)<<<total_tiles, gemm_st::THREADS, gemm_st::smem_bytes<1, 1>(), stream>>>(
-          probs_dev, tile_start_dev, nprob);
+      launch_chained(pick_tile_t<1, 1, 4>(ia, ib), total_tiles, gemm_st::THREADS, gemm_st::smem_bytes<1, 1>(), stream,
+                     probs_dev, tile_start_dev, nprob);
     return cudaGetLastError();
   }
-  pick_kernel(opA, opB, preload)<<<total_tiles, gemm::THREADS, gemm::SMEM_BYTES, stream>>>(probs_dev, tile_start_dev,
-                                                                                          nprob);
+  launch_chained(pick_kernel(opA, opB, preload), total_tiles, gemm::THREADS, gemm::SMEM_BYTES, stream, probs_dev,
+                 tile_start_dev, nprob);
   return cudaGetLastError();
 }
 
@@ -523,8 +525,8 @@ cudaError_t launch_zgemm_batched_ex(char opA, char opB, bool preload, const ZGem
 cudaError_t launch_zgemm_batched(char opA, char opB, const ZGemmProblem* probs_dev, const int* tile_start_dev,
                                  int nprob, int total_tiles, cudaStream_t stream) {
   if (nprob <= 0 || total_tiles <= 0) return cudaSuccess;
-  pick_kernel(opA, opB, false)<<<total_tiles, gemm::THREADS, gemm::SMEM_BYTES, stream>>>(
-      probs_dev, tile_start_dev, nprob);
+  launch_chained(pick_kernel(opA, opB, false), total_tiles, gemm::THREADS, gemm::SMEM_BYTES, stream, probs_dev,
+                 tile_start_dev, nprob);
   return cudaGetLastError();
 }
 

@@ -205,6 +205,7 @@ __device__ __forceinline__ void oz_digits(const OzSplitProblem& q, int e, int gr
 // per pass of 64 energies of 32 x 256): a third of the warps.
 template <int R>
 __global__ void __launch_bounds__(256, 5) ozaki_split1_kernel(const OzSplitProblem* __restrict__ probs, int ldt) {
+  chain_entry();
   const OzSplitProblem q = probs[blockIdx.y];
   const int r0 = blockIdx.x * R;
   if (r0 >= q.rows_pad) return;
@@ -264,6 +265,7 @@ __global__ void __launch_bounds__(256, 5) ozaki_split1_kernel(const OzSplitProbl
 }
 
 __global__ void __launch_bounds__(256, 3) ozaki_split_kernel(const OzSplitProblem* __restrict__ probs) {
+  chain_entry();
   const OzSplitProblem q = probs[blockIdx.y];
   const int r0 = blockIdx.x * oz::SPLIT_ROWS;
   if (r0 >= q.rows_pad) return;
@@ -517,6 +519,7 @@ template <int ND>
 __global__ void __launch_bounds__(oz::THREADS, 1)
     ozaki_mma_kernel(const OzMmaProblem* __restrict__ probs, const int4* __restrict__ tile_map, int total_tiles,
                      int* __restrict__ err, long long wait_cycles) {
+  chain_entry();
   using namespace oz;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], accf_bar, acce_bar, done_bar;
@@ -1061,15 +1064,15 @@ cudaError_t launch_ozaki_split(const void* probs, int nprob, int max_rows_pad, i
   const int R = split1_rows(max_k_pad);
   if (R == 0) {
     dim3 grid((max_rows_pad + oz::SPLIT_ROWS - 1) / oz::SPLIT_ROWS, nprob);
-    ozaki_split_kernel<<<grid, 256, kSplitSmem, st>>>(p);
+    launch_chained(ozaki_split_kernel, grid, 256, kSplitSmem, st, p);
     return cudaGetLastError();
   }
   // rows_pad is a multiple of 64, so of R; every problem's k_pad <= max_k_pad
   dim3 grid(max_rows_pad / R, nprob);
   const int ldt = max_k_pad + 1;
   const size_t smem = split1_smem(max_k_pad);
-  if (R == 16) ozaki_split1_kernel<16><<<grid, 256, smem, st>>>(p, ldt);
-  else ozaki_split1_kernel<8><<<grid, 256, smem, st>>>(p, ldt);
+  if (R == 16) launch_chained(ozaki_split1_kernel<16>, grid, 256, smem, st, p, ldt);
+  else launch_chained(ozaki_split1_kernel<8>, grid, 256, smem, st, p, ldt);
   return cudaGetLastError();
 }
 
@@ -1093,11 +1096,11 @@ cudaError_t launch_ozaki_mma(const void* probs, const void* tile_map, int total_
   const auto* pr = static_cast<const OzMmaProblem*>(probs);
   const auto* tm = static_cast<const int4*>(tile_map);
   if (pairs == 28)
-    ozaki_mma_kernel<7><<<grid, oz::THREADS, ozaki_mma_smem_bytes(), st>>>(pr, tm, total_tiles, err,
-                                                                           g_oz_wait_cycles.load());
+    launch_chained(ozaki_mma_kernel<7>, grid, oz::THREADS, ozaki_mma_smem_bytes(), st, pr, tm, total_tiles, err,
+                   g_oz_wait_cycles.load());
   else
-    ozaki_mma_kernel<8><<<grid, oz::THREADS, ozaki_mma_smem_bytes(), st>>>(pr, tm, total_tiles, err,
-                                                                           g_oz_wait_cycles.load());
+    launch_chained(ozaki_mma_kernel<8>, grid, oz::THREADS, ozaki_mma_smem_bytes(), st, pr, tm, total_tiles, err,
+                   g_oz_wait_cycles.load());
   return cudaGetLastError();
 }
 

@@ -80,6 +80,7 @@ __device__ __forceinline__ unsigned gj_key(double v, int row) {
 template <int T, int RT>
 __global__ void __launch_bounds__(T, 1)
     zgj_panel_kernel(const ZInvProblem* __restrict__ probs, GjPanelArgs args) {
+  chain_entry();
   using gj::SW;
   const ZInvProblem p = probs[blockIdx.x];
   const int n = p.n;
@@ -350,6 +351,7 @@ __global__ void __launch_bounds__(T, 1)
 // factoring warps with two rows per thread take 7 % longer at 100.
 template <int T>
 __global__ void __launch_bounds__(T, 512 / T) zgj_whole_kernel(const ZInvProblem* __restrict__ probs) {
+  chain_entry();
   using gj::SW;
   const ZInvProblem p = probs[blockIdx.x];
   const int n = p.n;
@@ -546,6 +548,7 @@ __global__ void __launch_bounds__(T, 512 / T) zgj_whole_kernel(const ZInvProblem
 template <int BN>
 __global__ void __launch_bounds__(256, 2)
     zgj_update_kernel(const ZInvProblem* __restrict__ probs, int k0, int nb, int stripes) {
+  chain_entry();
   constexpr int BM = 64, ALD = BM + 2, BLD = 36, NI = BN / 16;
   const int prob = blockIdx.x / stripes, c0 = (blockIdx.x - prob * stripes) * BN;
   const ZInvProblem& pp = probs[prob];
@@ -627,6 +630,7 @@ __global__ void __launch_bounds__(256, 2)
 // out[r, j] = W[piv[r], q[j]] with q the inverse permutation of piv:
 // out[r, piv[c]] = W[piv[r], c].
 __global__ void zgj_unpermute_kernel(const ZInvProblem* __restrict__ probs) {
+  chain_entry();
   const ZInvProblem p = probs[blockIdx.y];
   const int n = p.n;
   // one thread per (r, c) element of W's column c -> output column piv[c]
@@ -653,12 +657,12 @@ cudaError_t launch_zgj_panel(const ZInvProblem* probs_dev, int nprob, int k0, in
   if (nprob <= 0) return cudaSuccess;
   GjPanelArgs a{k0, nb, blocked};
   if (!blocked) {
-    if (max_n <= 32) zgj_whole_kernel<128><<<nprob, 128, smem, stream>>>(probs_dev);
-    else zgj_whole_kernel<256><<<nprob, 256, smem, stream>>>(probs_dev);
-  } else if (max_n <= 128) zgj_panel_kernel<128, 1><<<nprob, 128, smem, stream>>>(probs_dev, a);
-  else if (max_n <= 256) zgj_panel_kernel<256, 1><<<nprob, 256, smem, stream>>>(probs_dev, a);
-  else if (max_n <= 512) zgj_panel_kernel<256, 2><<<nprob, 256, smem, stream>>>(probs_dev, a);
-  else zgj_panel_kernel<256, 4><<<nprob, 256, smem, stream>>>(probs_dev, a);
+    if (max_n <= 32) launch_chained(zgj_whole_kernel<128>, nprob, 128, smem, stream, probs_dev);
+    else launch_chained(zgj_whole_kernel<256>, nprob, 256, smem, stream, probs_dev);
+  } else if (max_n <= 128) launch_chained(zgj_panel_kernel<128, 1>, nprob, 128, smem, stream, probs_dev, a);
+  else if (max_n <= 256) launch_chained(zgj_panel_kernel<256, 1>, nprob, 256, smem, stream, probs_dev, a);
+  else if (max_n <= 512) launch_chained(zgj_panel_kernel<256, 2>, nprob, 256, smem, stream, probs_dev, a);
+  else launch_chained(zgj_panel_kernel<256, 4>, nprob, 256, smem, stream, probs_dev, a);
   return cudaGetLastError();
 }
 
@@ -670,10 +674,12 @@ cudaError_t launch_zgj_update(const ZInvProblem* probs_dev, int nprob, int k0, i
   if (nprob <= 0) return cudaSuccess;
   const int s32 = (max_n + 31) / 32;
   if ((long long)nprob * s32 >= 2 * 148) {
-    zgj_update_kernel<32><<<nprob * s32, 256, zgj_update_smem_bytes(max_n, nb, 32), stream>>>(probs_dev, k0, nb, s32);
+    launch_chained(zgj_update_kernel<32>, nprob * s32, 256, zgj_update_smem_bytes(max_n, nb, 32), stream, probs_dev,
+                   k0, nb, s32);
   } else {
     const int s16 = (max_n + 15) / 16;
-    zgj_update_kernel<16><<<nprob * s16, 256, zgj_update_smem_bytes(max_n, nb, 16), stream>>>(probs_dev, k0, nb, s16);
+    launch_chained(zgj_update_kernel<16>, nprob * s16, 256, zgj_update_smem_bytes(max_n, nb, 16), stream, probs_dev,
+                   k0, nb, s16);
   }
   return cudaGetLastError();
 }
@@ -705,7 +711,7 @@ cudaError_t launch_zgj_unpermute(const ZInvProblem* probs_dev, int nprob, int ma
   int bx = (per + 255) / 256;
   if (bx > 64) bx = 64;
   dim3 grid(bx, nprob);
-  zgj_unpermute_kernel<<<grid, 256, 0, stream>>>(probs_dev);
+  launch_chained(zgj_unpermute_kernel, grid, 256, 0, stream, probs_dev);
   return cudaGetLastError();
 }
 

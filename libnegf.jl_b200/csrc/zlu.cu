@@ -28,6 +28,7 @@ constexpr int LU_THREADS = 256;
 
 __global__ void __launch_bounds__(LU_THREADS)
     zgetrf_panel_kernel(const ZLuProblem* __restrict__ probs, int k0, int nb) {
+  chain_entry();
   const ZLuProblem p = probs[blockIdx.x];
   const int n = p.n;
   if (k0 >= n) return;
@@ -119,6 +120,7 @@ __global__ void __launch_bounds__(LU_THREADS)
 // Row interchanges of panel [k0, k0+w) on every column outside the panel,
 // then T = A[k0:k0+w, k0+w:n] (w x (n-k0-w), ld w).
 __global__ void zlaswp_copy_kernel(const ZLuProblem* __restrict__ probs, int k0, int nb) {
+  chain_entry();
   const ZLuProblem p = probs[blockIdx.y];
   const int n = p.n;
   if (k0 >= n) return;
@@ -143,6 +145,7 @@ __global__ void zlaswp_copy_kernel(const ZLuProblem* __restrict__ probs, int k0,
 // upper -> inverse of the non-unit upper triangle, else the inverse of the
 // unit lower triangle.  X is the n x n output (zero elsewhere beforehand).
 __global__ void ztrtri_diag_kernel(const ZTriProblem* __restrict__ probs, int nb, int upper) {
+  chain_entry();
   const ZTriProblem p = probs[blockIdx.y];
   const int j0 = blockIdx.x * nb;
   if (j0 >= p.n) return;
@@ -198,6 +201,7 @@ __global__ void ztrtri_diag_kernel(const ZTriProblem* __restrict__ probs, int nb
 constexpr int kLuDiag = 32;
 __global__ void __launch_bounds__(256)
     zlu_diag_kernel(const ZLuDiagProblem* __restrict__ probs, int k0) {
+  chain_entry();
   const ZLuDiagProblem p = probs[blockIdx.x];
   if (k0 >= p.n) return;
   constexpr int LD = kLuDiag + 1;
@@ -255,6 +259,7 @@ __global__ void __launch_bounds__(256)
 // would be faster, but without row interchanges U may have small pivots: the
 // selected inverse of NEGF matrices lost a digit.)
 __global__ void __launch_bounds__(64) zlu_solve_kernel(const ZLuDiagProblem* __restrict__ probs, int k0, int chunks) {
+  chain_entry();
   const ZLuDiagProblem p = probs[blockIdx.y];
   const int k1 = k0 + kLuDiag;
   const bool rows = (int)blockIdx.x < chunks;
@@ -310,14 +315,15 @@ cudaError_t launch_zlu_solve(const void* probs, int nprob, int k0, int max_n, cu
   const int chunks = (rest + 63) / 64;
   for (int base = 0; base < nprob; base += 65535) {  // grid.y is limited to 65535
     const int cnt = nprob - base < 65535 ? nprob - base : 65535;
-    zlu_solve_kernel<<<dim3(2 * chunks, cnt), 64, 0, st>>>(static_cast<const ZLuDiagProblem*>(probs) + base, k0, chunks);
+    launch_chained(zlu_solve_kernel, dim3(2 * chunks, cnt), 64, 0, st,
+                   static_cast<const ZLuDiagProblem*>(probs) + base, k0, chunks);
   }
   return cudaGetLastError();
 }
 
 cudaError_t launch_zlu_diag(const void* probs, int nprob, int k0, cudaStream_t st) {
   if (nprob <= 0) return cudaSuccess;
-  zlu_diag_kernel<<<nprob, 256, 0, st>>>(static_cast<const ZLuDiagProblem*>(probs), k0);
+  launch_chained(zlu_diag_kernel, nprob, 256, 0, st, static_cast<const ZLuDiagProblem*>(probs), k0);
   return cudaGetLastError();
 }
 
@@ -344,14 +350,14 @@ cudaError_t zlu_prepare(size_t panel_smem, size_t tri_smem) {
 
 cudaError_t launch_zgetrf_panel(const void* probs, int nprob, int k0, int nb, size_t smem, cudaStream_t st) {
   if (nprob <= 0) return cudaSuccess;
-  zgetrf_panel_kernel<<<nprob, LU_THREADS, smem, st>>>(static_cast<const ZLuProblem*>(probs), k0, nb);
+  launch_chained(zgetrf_panel_kernel, nprob, LU_THREADS, smem, st, static_cast<const ZLuProblem*>(probs), k0, nb);
   return cudaGetLastError();
 }
 
 cudaError_t launch_zlaswp_copy(const void* probs, int nprob, int k0, int nb, int max_n, cudaStream_t st) {
   if (nprob <= 0) return cudaSuccess;
   dim3 grid((max_n + 127) / 128, nprob);
-  zlaswp_copy_kernel<<<grid, 128, 0, st>>>(static_cast<const ZLuProblem*>(probs), k0, nb);
+  launch_chained(zlaswp_copy_kernel, grid, 128, 0, st, static_cast<const ZLuProblem*>(probs), k0, nb);
   return cudaGetLastError();
 }
 
@@ -359,7 +365,7 @@ cudaError_t launch_ztrtri_diag(const void* probs, int nprob, int nb, int upper, 
                                cudaStream_t st) {
   if (nprob <= 0) return cudaSuccess;
   dim3 grid((max_n + nb - 1) / nb, nprob);
-  ztrtri_diag_kernel<<<grid, 64, smem, st>>>(static_cast<const ZTriProblem*>(probs), nb, upper);
+  launch_chained(ztrtri_diag_kernel, grid, 64, smem, st, static_cast<const ZTriProblem*>(probs), nb, upper);
   return cudaGetLastError();
 }
 
