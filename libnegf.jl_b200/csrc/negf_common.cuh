@@ -50,7 +50,8 @@ __host__ __device__ inline cplx cinv(cplx a) {
   }
 }
 #ifdef __CUDACC__
-// 1/a (0 for a = 0, and for infinite a).  a is scaled by a power of two
+// 1/a; 0 for a = 0 and where one part is infinite and the other finite, NaN for
+// any other non-finite a, as cinv gives.  a is scaled by a power of two
 // (exact), so that d = |a|^2 lies within [2^-102, 32); 1/d starts from a
 // single-precision reciprocal and takes one third-order Newton-Raphson step,
 // x (1 + e + e^2) with e = 1 - d x: |e| < 2^-21, so the step's error e^3 is
@@ -67,7 +68,11 @@ __device__ __forceinline__ cplx cinv_pivot(cplx a) {
   const double x0 = xf;
   const double r = fma(-d, x0, 1.0);
   const double t = fma(x0, fma(r, r, r), x0);
-  const bool none = (hx | hy | __double2loint(a.x) | __double2loint(a.y)) == 0 || e == 0x7ff;
+  const int lx = __double2loint(a.x), ly = __double2loint(a.y);
+  // the parts' high words tell infinity (0x7ff00000, low word 0) from NaN; with
+  // x0 = 1 / infinity = 0 every other non-finite a turns r, and so t, into NaN
+  const bool inf1 = max(hx, hy) == 0x7ff00000 && (hx > hy ? lx : ly) == 0 && min(hx, hy) < 0x7ff00000;
+  const bool none = (hx | hy | lx | ly) == 0 || inf1;
   return none ? make_double2(0.0, 0.0) : make_double2(x * t * s, -y * t * s);
 }
 

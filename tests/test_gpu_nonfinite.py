@@ -1,0 +1,52 @@
+"""NaN and infinities never come back as a success with finite numbers."""
+
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+BAD = {"nan": complex(np.nan, 0.0), "nan_im": complex(0.0, np.nan), "inf_inf": complex(np.inf, -np.inf),
+       "inf_nan": complex(np.inf, np.nan)}
+
+
+def _mat(rng, n):
+    return rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+
+
+def _device(negf, npl, b):
+    rng = np.random.default_rng(npl * b)
+    Hd, Hu = [], []
+    for _ in range(npl):
+        A = _mat(rng, b) / np.sqrt(2 * b)
+        Hd.append((A + A.conj().T) / 2)
+    for _ in range(npl - 1):
+        Hu.append(0.25 * _mat(rng, b) / np.sqrt(b))
+    s = -0.05j * np.eye(b)
+    return negf.Device(Hd, Hu, s, s)
+
+
+@pytest.mark.parametrize("bad", sorted(BAD))
+@pytest.mark.parametrize("n", [1, 20, 33, 70, 150])
+def test_unpivoted_lu(negf, n, bad):
+    """A non-finite pivot reaches every element of the block's inverse."""
+    from libnegf_b200._lib import ptr_array
+    rng = np.random.default_rng(n)
+    for i, j in {(0, 0), (n // 2, n // 2), (n - 1, n - 1), (n - 1, 0)}:
+        a = _mat(rng, n) + 3.0 * n * np.eye(n)
+        a[i, j] = BAD[bad]
+        d, fill = negf.to_device(a), (ctypes.c_uint8 * 1)()
+        rc = negf.load().negf_selected_inverse_batched(1, 1, n, ptr_array([d.data_ptr()]), fill, 3, 0, 0, None)
+        assert rc != 0 or np.isnan(negf.to_host(d)).all()
+
+
+@pytest.mark.parametrize("npl,b", [(3, 24), (3, 70)])
+def test_selected_inverse_nan_energy(negf, npl, b):
+    """The energies beside a NaN are not touched by it."""
+    d = _device(negf, npl, b)
+    alone = d.selected_inverse([0.1], "selinv", eta=1e-2)
+    both = d.selected_inverse([0.1, np.nan], "selinv", eta=1e-2)
+    for x, y in zip(alone, both):
+        assert all(np.array_equal(p, q) for p, q in zip(x[0], y[0]))
+        assert all(np.isnan(q).all() for q in y[1])
