@@ -129,7 +129,8 @@ __global__ void __launch_bounds__(T, 1)
         const int r = tid + k * T;
         a[k][j] = (r < n && j < sw) ? S[(size_t)(s0 + j) * ldw + r] : make_double2(0.0, 0.0);
       }
-    // candidate of the current column: this thread's key (NaN rows never qualify) and entry
+    // candidate of the current column: this thread's key (NaN rows never qualify; an
+    // arithmetic NaN may carry a sign, so the comparison is unsigned) and entry
     unsigned key = 0, wkey = 0;
     cplx cand = make_double2(0.0, 0.0);
     auto search = [&] {
@@ -137,7 +138,7 @@ __global__ void __launch_bounds__(T, 1)
 #pragma unroll
       for (int k = 0; k < RT; ++k) {
         const double v = cabs1(a[k][0]);
-        const unsigned q = !used[k] && __double2hiint(v) <= 0x7ff00000 ? gj_key(v, tid + k * T) : 0u;
+        const unsigned q = !used[k] && (unsigned)__double2hiint(v) <= 0x7ff00000u ? gj_key(v, tid + k * T) : 0u;
         if (q > key) {
           key = q;
           cand = a[k][0];
@@ -398,7 +399,7 @@ __global__ void __launch_bounds__(T, 512 / T) zgj_whole_kernel(const ZInvProblem
     unsigned key = 0, wkey = 0;
     auto search = [&] {
       const double v = cabs1(a[0]);
-      key = !used && __double2hiint(v) <= 0x7ff00000 ? gj_key(v, ptid) : 0u;
+      key = !used && (unsigned)__double2hiint(v) <= 0x7ff00000u ? gj_key(v, ptid) : 0u;
       wkey = __reduce_max_sync(0xffffffffu, key);
     };
     search();

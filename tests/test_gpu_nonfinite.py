@@ -50,3 +50,25 @@ def test_selected_inverse_nan_energy(negf, npl, b):
     for x, y in zip(alone, both):
         assert all(np.array_equal(p, q) for p, q in zip(x[0], y[0]))
         assert all(np.isnan(q).all() for q in y[1])
+
+
+@pytest.mark.parametrize("bad", sorted(BAD))
+@pytest.mark.parametrize("n", [1, 8, 40, 100, 140, 300, 520])
+def test_inversion(negf, n, bad):
+    """The Gauss-Jordan kernels report a matrix whose rows turn into NaN: NaN
+    rows are never pivots, so a later column has no candidate left."""
+    from libnegf_b200._lib import NEGF_ERR_SINGULAR, int_array, ptr_array
+    rng = np.random.default_rng(n)
+    good = _mat(rng, n)
+    for i, j in {(0, 0), (n // 2, n // 2), (n - 1, 0), (0, n - 1)}:
+        a = good.copy()
+        a[i, j] = BAD[bad]
+        dA, dO = [negf.to_device(x) for x in (good, a)], [negf.dzeros(n, n) for _ in range(2)]
+        info = (ctypes.c_int32 * 2)()
+        rc = negf.load().negf_zinv_batched(2, int_array([n, n]), ptr_array([x.data_ptr() for x in dA]), int_array([n, n]),
+                                           ptr_array([x.data_ptr() for x in dO]), int_array([n, n]), info, None)
+        assert info[0] == 0
+        if n > 1:
+            assert rc == NEGF_ERR_SINGULAR and info[1] > 0
+        else:
+            assert rc == NEGF_ERR_SINGULAR or np.isnan(negf.to_host(dO[1])).all()
