@@ -336,8 +336,8 @@ int negf_solve(negf_device_t dev, int32_t nE, const double* energies, const negf
  *             size).
  * opts: eta, precision (NEGF_PREC_MIXED: block products on the INT8 tensor
  * cores with FP64-grade digit splitting, inversion panels and LU in FP64),
- * max_chunk / hbm_budget_gb (energies per chunk), gemm_form, gj_nb,
- * gj_update; sigma_per_energy must
+ * max_chunk / hbm_budget_gb (energies per chunk), gemm_form, gj_nb (any width
+ * that fits shared memory; taken in steps of 8 and up to 32), gj_update; sigma_per_energy must
  * be 0.  Outputs (NULL: skipped), energy-major: gd_out nE * sum b_i^2; gu_out
  * (blocks (i,i+1), b_i x b_{i+1}) and gl_out (blocks (i+1,i), b_{i+1} x b_i)
  * nE * sum b_i b_{i+1}; column-major blocks.  HOST pointers unless

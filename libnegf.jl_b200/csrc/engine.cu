@@ -43,9 +43,13 @@ int gj_panel_width(int max_n) {
   return 8;
 }
 
+// A requested width is taken in whole sub-panels of 8 (a partial one costs as
+// much shared memory) and up to the widest that the update kernel holds; the
+// inverse does not depend on it beyond rounding.
 int Plan::panel_width(int max_n) const {
-  if (gj_nb_ > 0 && max_n > 112) return gj_nb_;
-  return gj_panel_width(max_n);
+  if (gj_nb_ <= 0 || max_n <= 112) return gj_panel_width(max_n);
+  const int nb = std::min(gj_nb_, kGjMaxNb);
+  return nb < 8 ? nb : nb & ~7;
 }
 
 int TriSystem::maxb() const {

@@ -208,6 +208,17 @@ size_t max_panel_smem() {
   return (size_t)v;
 }
 
+// A panel of gj_nb columns with a column and a row beside it fits the shared
+// memory of a block, for every block of the device that is inverted in panels.
+bool gj_nb_fits(const negf_device_s& d, int gj_nb) {
+  if (gj_nb <= 0) return true;
+  for (int x : d.b) {
+    const size_t n = x, w = std::min(x, gj_nb);
+    if (x > 112 && (n * w + n + w) * sizeof(cplx) + 4 * w + n + 192 > max_panel_smem()) return false;
+  }
+  return true;
+}
+
 // One plan for every (device, energy) item of the batch: the devices may differ
 // in layer count and block sizes; each batched launch takes the items whose
 // recursion reaches that step. Item e uses parameter slots e (shift), nE + e
@@ -254,9 +265,8 @@ int build_solver(negf_solver_s& S) {
   if (S.opts.gj_nb != 0 && S.opts.gj_nb != 8 && S.opts.gj_nb != 16 && S.opts.gj_nb != 32)
     return fail(NEGF_ERR_INVALID, "gj_nb must be 0, 8, 16 or 32");
   for (negf_device_s* dv : S.devs)
-    for (int x : dv->b)
-      if (S.opts.gj_nb > 0 && x > 112 && zgj_panel_smem_bytes(x, S.opts.gj_nb) > max_panel_smem())
-        return fail(NEGF_ERR_INVALID, "gj_nb too wide for the block size (shared memory)");
+    if (!gj_nb_fits(*dv, S.opts.gj_nb))
+      return fail(NEGF_ERR_INVALID, "gj_nb too wide for the block size (shared memory)");
   if (S.opts.gj_update < 0 || S.opts.gj_update > 2) return fail(NEGF_ERR_INVALID, "gj_update must be 0, 1 or 2");
   plan.set_schedule(S.opts.gemm_form, S.opts.gj_nb);
   plan.set_fixed_order(true);  // chunks, batches and server groups of any size agree
@@ -1235,6 +1245,8 @@ int negf_device_selected_inverse(negf_device_t dev, int32_t nE, const double* en
   if (opts->sigma_per_energy)
     return fail(NEGF_ERR_INVALID, "negf_device_selected_inverse: the device's constant self-energies are used");
   const negf_device_s& d = *dev;
+  if (method != 2 && !gj_nb_fits(d, opts->gj_nb))
+    return fail(NEGF_ERR_INVALID, "negf_device_selected_inverse: gj_nb too wide for the block size (shared memory)");
   const int n = d.npl;
   int mb = 0;
   for (int x : d.b) mb = std::max(mb, x);

@@ -157,6 +157,9 @@ struct ZInvProblem {
   int n, ld, ldo, pad_;
 };
 
+// Widest Gauss-Jordan panel: the pivot-row buffer of zgj_update_kernel.
+constexpr int kGjMaxNb = 32;
+
 // One matrix of a batched LU (zlu.cu).
 struct ZLuProblem {
   cplx* A;       // n x n, ld

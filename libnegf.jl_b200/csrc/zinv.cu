@@ -550,7 +550,7 @@ template <int BN>
 __global__ void __launch_bounds__(256, 2)
     zgj_update_kernel(const ZInvProblem* __restrict__ probs, int k0, int nb, int stripes) {
   chain_entry();
-  constexpr int BM = 64, ALD = BM + 2, BLD = 36, NI = BN / 16;
+  constexpr int BM = 64, ALD = BM + 2, BLD = kGjMaxNb + 4, NI = BN / 16;
   const int prob = blockIdx.x / stripes, c0 = (blockIdx.x - prob * stripes) * BN;
   const ZInvProblem& pp = probs[prob];
   const int n = pp.n, ld = pp.ld;
@@ -668,11 +668,12 @@ cudaError_t launch_zgj_panel(const ZInvProblem* probs_dev, int nprob, int k0, in
 }
 
 static size_t zgj_update_smem_bytes(int max_n, int nb, int bn) {
-  return (2 * (size_t)((nb + 3) & ~3) * 66 + (size_t)bn * 36) * sizeof(cplx) + ((max_n + 15) & ~15);
+  return (2 * (size_t)((nb + 3) & ~3) * 66 + (size_t)bn * (kGjMaxNb + 4)) * sizeof(cplx) + ((max_n + 15) & ~15);
 }
 
 cudaError_t launch_zgj_update(const ZInvProblem* probs_dev, int nprob, int k0, int nb, int max_n, cudaStream_t stream) {
   if (nprob <= 0) return cudaSuccess;
+  if (nb > kGjMaxNb) return cudaErrorInvalidValue;
   const int s32 = (max_n + 31) / 32;
   if ((long long)nprob * s32 >= 2 * 148) {
     launch_chained(zgj_update_kernel<32>, nprob * s32, 256, zgj_update_smem_bytes(max_n, nb, 32), stream, probs_dev,
