@@ -50,13 +50,15 @@ __device__ __forceinline__ void gj_dmma(double (&c)[4], double a0, double a1, do
 }
 
 // Pivot candidates compare as 32-bit keys: the leading 21 bits of |re| + |im|
-// (exponent and 10 mantissa bits; plus 1, so that 0 means no candidate) over
-// 1023 - row, so that one REDUX gives value and row.  The pivot is within 0.1 %
-// of the largest |re| + |im| of its column, the lowest row among those that
-// share the leading bits; the growth bound of partial pivoting changes by that
-// factor only.
+// (exponent and 10 mantissa bits) in the upper 22, over 1023 - row, so that one
+// REDUX gives value and row.  The upper part is 0 without a candidate, 1 for an
+// exact zero and larger for every other value.  The pivot is within 0.1 % of the
+// largest |re| + |im| of its column, the lowest row among those that share the
+// leading bits; the growth bound of partial pivoting changes by that factor only.
+// (Values below 2^-1032 all share them; the reciprocal of each overflows.)
 __device__ __forceinline__ unsigned gj_key(double v, int row) {
-  return ((((unsigned)__double2hiint(v) >> 10) + 1u) << 10) | (unsigned)(1023 - row);
+  const unsigned hi = __double2hiint(v);
+  return (((hi >> 10) + ((hi | (unsigned)__double2loint(v)) != 0u ? 2u : 1u)) << 10) | (unsigned)(1023 - row);
 }
 
 // Gauss-Jordan on an n x w slab held in shared memory (column-major, odd
@@ -175,17 +177,15 @@ __global__ void __launch_bounds__(T, 1)
         }
       }
       const int pr = 1023 - (int)(best & 1023u);
-      if (best < 2048u) {  // no candidate row, or one whose leading bits are zero (uniform)
+      if (best < 2048u) {  // no candidate row, or zeros only (uniform)
+        if (tid == 0 && p.info) atomicCAS(p.info, 0, k0 + s0 + j + 1);
         if (best == 0u) {
           if (tid == 0) {
             *sh_dead = 1;
             sh_piv[s0 + j] = -1;
-            if (p.info) atomicCAS(p.info, 0, k0 + s0 + j + 1);
           }
           break;
         }
-        const cplx x = slot[(buf + ((pr % T) >> 5)) * SW];  // 0 for a zero pivot
-        if (tid == 0 && p.info && x.x == 0.0 && x.y == 0.0) atomicCAS(p.info, 0, k0 + s0 + j + 1);
       }
       const cplx* row = slot + (buf + ((pr % T) >> 5)) * SW;
       if (tid == pw * 32 - 1) {
@@ -423,15 +423,12 @@ __global__ void __launch_bounds__(T, 512 / T) zgj_whole_kernel(const ZInvProblem
       }
       const int pr = 1023 - (int)(best & 1023u);
       const cplx* row = slot + (buf + (pr % PT >> 5)) * SW;
-      if (best < 2048u) {  // no candidate row, or one whose leading bits are zero (uniform)
+      if (best < 2048u) {  // no candidate row, or zeros only (uniform)
+        if (ptid == 0 && p.info) atomicCAS(p.info, 0, s0 + j + 1);
         if (best == 0u) {
-          if (ptid == 0) {
-            *sh_dead = 1;
-            if (p.info) atomicCAS(p.info, 0, s0 + j + 1);
-          }
+          if (ptid == 0) *sh_dead = 1;
           break;
         }
-        if (ptid == 0 && p.info && row[0].x == 0.0 && row[0].y == 0.0) atomicCAS(p.info, 0, s0 + j + 1);
       }
       if (ptid == PT - 1) {
         sh_piv[s0 + j] = pr;

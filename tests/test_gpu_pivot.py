@@ -22,3 +22,20 @@ def test_reciprocal(negf, scale, ratio):
     d = x * x + y * y
     for g, r in ((got.real, x / d), (got.imag, -y / d)):
         assert np.all(np.abs(g - r) <= 1.02 * 2.0 ** -53 * np.abs(r))
+
+
+@pytest.mark.parametrize("n", [2, 40, 100, 140, 300])
+@pytest.mark.parametrize("tiny", [5e-324, 1e-320, 1e-312])
+def test_tiny_pivot_is_not_zero(negf, n, tiny):
+    """A column of zeros and one subnormal entry has a pivot; its reciprocal
+    overflows, so the call may fail in a later column, but not in this one."""
+    from libnegf_b200._lib import int_array, ptr_array
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    a[:, 0] = 0.0
+    a[n // 2, 0] = tiny
+    d, o, info = negf.to_device(a), negf.dzeros(n, n), (ctypes.c_int32 * 1)()
+    negf.load().negf_zinv_batched(1, int_array([n]), ptr_array([d.data_ptr()]), int_array([n]), ptr_array([o.data_ptr()]),
+                                  int_array([n]), info, None)
+    assert info[0] != 1
+    assert info[0] > 1 or not np.isfinite(negf.to_host(o)).all()
