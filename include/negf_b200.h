@@ -63,7 +63,9 @@ typedef struct {
 } negf_zgemm_problem;
 
 /* Batched be_gemm! (src/backend_cpu.jl:208-219): all problems share
- * opA, opB in {'N','T','C'}.  One launch on the FP64 tensor path. */
+ * opA, opB in {'N','T','C'}.  One launch on the FP64 tensor path, in tiles that
+ * follow the amount of work in the call: the last bits of a result may depend on
+ * the number of problems (as for the sweeps of single systems below). */
 int negf_zgemm_batched(char opA, char opB, int32_t nprob, const negf_zgemm_problem* probs, void* stream);
 
 /* negf_zgemm_batched in the MIXED precision mode (INT8 tensor cores with

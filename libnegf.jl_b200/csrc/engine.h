@@ -189,8 +189,10 @@ class Plan {
   // schedule knobs: FP64 GEMM form (0 default, 1 four products, 2 3M) and the
   // Gauss-Jordan panel width for blocks > 112 (0 default)
   void set_schedule(int gemm_form, int gj_nb) { gemm_form_ = gemm_form; gj_nb_ = gj_nb; }
-  // FP64 products add in an order that does not depend on the other problems of
-  // their step: a system's results are the same whatever batch it is solved in
+  // FP64 products (default form) add in an order that does not depend on the other
+  // problems of their step.  Inversions take their form and panel width from the
+  // largest block of a step, so a system's results are the same to the last bit
+  // beside any number of systems with its block sizes, not beside larger blocks.
   void set_fixed_order(bool on) { fixed_order_ = on; }
   // Gauss-Jordan rank-nb updates of a mixed plan: 1 FP64 DMMA products, 2
   // INT8 digit products with 34 pairs (as accurate as FP64 products), 0 the

@@ -269,7 +269,7 @@ int build_solver(negf_solver_s& S) {
       return fail(NEGF_ERR_INVALID, "gj_nb too wide for the block size (shared memory)");
   if (S.opts.gj_update < 0 || S.opts.gj_update > 2) return fail(NEGF_ERR_INVALID, "gj_update must be 0, 1 or 2");
   plan.set_schedule(S.opts.gemm_form, S.opts.gj_nb);
-  plan.set_fixed_order(true);  // chunks, batches and server groups of any size agree
+  plan.set_fixed_order(true);  // the same energy agrees in chunks and batches of any number of energies
   plan.set_gj_update(S.opts.gj_update);
 
   const bool sig_e = S.opts.sigma_per_energy != 0;
