@@ -44,6 +44,8 @@
 // returns, and the host reports the error.
 #include "negf_common.cuh"
 
+#include <math_constants.h>
+
 #include <atomic>
 #include <cstdint>
 #include <vector>
@@ -73,6 +75,9 @@ constexpr int TMEM_COLS = 512;          // ND_MAX x TN
 static_assert(TMEM_COLS == ND_MAX * TN, "one accumulator per digit diagonal");
 constexpr long long WAIT_CYCLES = 2000000000LL;  // ~1 s at 1.9 GHz per wait
 constexpr int SPLIT_ROWS = 64;          // rows per split CTA
+// exponent of an operand row with a NaN or an infinity: it has no digits, and the
+// product kernel writes NaN in its row or column of C (finite rows: -1073 .. 1024)
+constexpr int BAD_ROW = 1 << 14;
 // offset that turns the six lower bytes of x + C6 into digits + 128:
 // C6 = 128 (256^6 - 1) / 255
 constexpr long long C6 = 128LL * ((1LL << 48) - 1) / 255;
@@ -237,20 +242,32 @@ __global__ void __launch_bounds__(256, 5) ozaki_split1_kernel(const OzSplitProbl
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
-  // row maxima of |re| + |im| (bounds |re|, |im| and |re + im|), a warp per row
+  // row maxima of |re| + |im| (bounds |re|, |im| and |re + im|), a warp per row:
+  // the exponent is in the largest high word (as an unsigned number: a NaN of
+  // either sign and infinity are the largest), but for subnormal rows
   for (int r = warp; r < R; r += 8) {
-    double mx = 0.0;
+    unsigned hm = 0u;
     for (int k = lane; k < kp; k += 32) {
       const cplx v = tile[(size_t)r * ldt + k];
-      mx = fmax(mx, fabs(v.x) + fabs(v.y));
+      hm = max(hm, (unsigned)__double2hiint(fabs(v.x) + fabs(v.y)));
     }
+    hm = __reduce_max_sync(0xffffffffu, hm);
+    int e = (int)(hm >> 20) - 1022;  // max < 2^e
+    if (hm < 0x00100000u) {
+      double mx = 0.0;
+      for (int k = lane; k < kp; k += 32) {
+        const cplx v = tile[(size_t)r * ldt + k];
+        mx = fmax(mx, fabs(v.x) + fabs(v.y));
+      }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      e = 0;
+      if (mx > 0.0) frexp(mx, &e);
+    }
     if (lane == 0) {
-      int e = 0;
-      if (mx > 0.0) frexp(mx, &e);  // mx < 2^e
-      sh_e[r] = e;
-      q.exps[r0 + r] = e;
+      const bool bad = hm >= 0x7ff00000u;
+      sh_e[r] = bad ? 0 : e;
+      q.exps[r0 + r] = bad ? oz::BAD_ROW : e;
     }
   }
   __syncthreads();
@@ -263,6 +280,9 @@ __global__ void __launch_bounds__(256, 5) ozaki_split1_kernel(const OzSplitProbl
     oz_digits(q, sh_e[rl], r0 + rl, kq, c, tile + (size_t)rl * ldt + c * oz::KC + 4 * kq);
   }
 }
+
+// the larger of m and v; infinity for a NaN v
+__device__ __forceinline__ double oz_max(double m, double v) { return isnan(v) ? CUDART_INF : fmax(m, v); }
 
 __global__ void __launch_bounds__(256, 3) ozaki_split_kernel(const OzSplitProblem* __restrict__ probs) {
   chain_entry();
@@ -287,16 +307,17 @@ __global__ void __launch_bounds__(256, 3) ozaki_split_kernel(const OzSplitProble
 #pragma unroll 4
       for (int k = tid >> 6; k < q.cols; k += 4) {
         const cplx v = q.X[(long long)gr + (long long)k * q.sk];
-        mx = fmax(mx, fabs(v.x) + fabs(v.y));
+        mx = oz_max(mx, fabs(v.x) + fabs(v.y));
       }
     red[tid >> 6][r] = mx;
     __syncthreads();
     if (tid < oz::SPLIT_ROWS) {
       const double m = fmax(fmax(red[0][tid], red[1][tid]), fmax(red[2][tid], red[3][tid]));
+      const bool bad = isinf(m);
       int e = 0;
-      if (m > 0.0) frexp(m, &e);  // m < 2^e
+      if (m > 0.0 && !bad) frexp(m, &e);  // m < 2^e
       sh_e[tid] = e;
-      q.exps[r0 + tid] = e;
+      q.exps[r0 + tid] = bad ? oz::BAD_ROW : e;
     }
   } else {
     for (int j = 0; j < 8; ++j) {
@@ -306,15 +327,16 @@ __global__ void __launch_bounds__(256, 3) ozaki_split_kernel(const OzSplitProble
 #pragma unroll 4
         for (int k = lane; k < q.cols; k += 32) {
           const cplx v = q.X[(long long)gr * q.sr + k];
-          mx = fmax(mx, fabs(v.x) + fabs(v.y));
+          mx = oz_max(mx, fabs(v.x) + fabs(v.y));
         }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
       if (lane == 0) {
+        const bool bad = isinf(mx);
         int e = 0;
-        if (mx > 0.0) frexp(mx, &e);
+        if (mx > 0.0 && !bad) frexp(mx, &e);
         sh_e[r] = e;
-        q.exps[r0 + r] = e;
+        q.exps[r0 + r] = bad ? oz::BAD_ROW : e;
       }
     }
   }
@@ -783,8 +805,8 @@ __global__ void __launch_bounds__(oz::THREADS, 1)
             xr = cr[j] * sc;
             xi = ci[j] * sc;
           } else {
-            xr = ldexp(cr[j], e);
-            xi = ldexp(ci[j], e);
+            xr = e < BAD_ROW / 2 ? ldexp(cr[j], e) : CUDART_NAN;
+            xi = e < BAD_ROW / 2 ? ldexp(ci[j], e) : CUDART_NAN;
           }
           cplx v;
           if (has_cin) {

@@ -72,3 +72,45 @@ def test_inversion(negf, n, bad):
             assert rc == NEGF_ERR_SINGULAR and info[1] > 0
         else:
             assert rc == NEGF_ERR_SINGULAR or np.isnan(negf.to_host(dO[1])).all()
+
+
+@pytest.mark.parametrize("bad", sorted(BAD) + ["inf"])
+@pytest.mark.parametrize("ops", ["NN", "TC", "CT"])
+@pytest.mark.parametrize("k", [20, 130, 300, 600])
+def test_mixed_product(negf, ops, k, bad):
+    """A bad element of op(A) or op(B) makes its row or column of the result NaN
+    and leaves the rest to the last bit."""
+    rng = np.random.default_rng(k)
+    m, n = 70, 45
+    v = BAD.get(bad, complex(-np.inf, 1.0))
+    op = {"N": lambda x: x, "T": lambda x: x.T, "C": lambda x: x.conj().T}
+    A, B, C = _mat(rng, k)[:m].copy() if k >= m else _mat(rng, m)[:, :k].copy(), _mat(rng, max(k, n))[:k, :n].copy(), \
+        _mat(rng, m)[:, :n].copy()
+
+    def run(a, b):
+        out = negf.to_device(C.copy())
+        negf.be_gemm_batched_(ops[0], ops[1], [(1.0 - 0.5j, negf.to_device(np.ascontiguousarray(op[ops[0]](a))),
+                                                negf.to_device(np.ascontiguousarray(op[ops[1]](b))), 1.0, out)], "mixed")
+        return negf.to_host(out)
+
+    clean = run(A, B)
+    assert np.isfinite(clean).all()
+    for i in (0, 33, m - 1):
+        X = A.copy()
+        X[i, k // 2] = v
+        got = run(X, B)
+        rest = np.arange(m) != i
+        assert np.isnan(got[i]).all() and np.array_equal(got[rest], clean[rest])
+    for j in (0, 17, n - 1):
+        Y = B.copy()
+        Y[k - 1, j] = v
+        got = run(A, Y)
+        rest = np.arange(n) != j
+        assert np.isnan(got[:, j]).all() and np.array_equal(got[:, rest], clean[:, rest])
+
+
+def test_mixed_selected_inverse_nan_energy(negf):
+    d = _device(negf, 3, 130)
+    r = d.selected_inverse([0.1, np.nan], "selinv", "mixed", eta=1e-2)
+    for x in r:
+        assert all(np.isfinite(q).all() for q in x[0]) and all(np.isnan(q).all() for q in x[1])
