@@ -216,15 +216,17 @@ __global__ void __launch_bounds__(256)
     S[j * LD + r] = r < w && j < w ? p.A[(k0 + r) + (size_t)(k0 + j) * p.ld] : one;
     Y[j * LD + r] = one;
   }
+  // reciprocal of pivot c, by the thread of that element as soon as it is final:
+  // in every thread the reciprocals would load the FP64 pipe as much as the updates
+  auto pivot = [&](int c) {
+    const cplx piv = S[c * LD + c];
+    inv[c] = cinv_pivot(piv);
+    if (piv.x == 0.0 && piv.y == 0.0 && p.info) atomicCAS(p.info, 0, k0 + c + 1);
+  };
+  if (threadIdx.x == 0) pivot(0);
   __syncthreads();
   for (int c = 0; c < w; ++c) {
-    const cplx piv = S[c * LD + c];
-    const bool zero = piv.x == 0.0 && piv.y == 0.0;
-    const cplx iv = cinv_pivot(piv);
-    if (threadIdx.x == 0) {
-      inv[c] = iv;
-      if (zero && p.info) atomicCAS(p.info, 0, k0 + c + 1);
-    }
+    const cplx iv = inv[c];
     if (r > c) {
       const cplx l = cmul(S[c * LD + r], iv);
 #pragma unroll
@@ -232,6 +234,7 @@ __global__ void __launch_bounds__(256)
         const int m = j * LD + (j > c ? 0 : YO);
         S[m + r] = cfms_fused(S[m + r], l, S[m + c]);
       }
+      if (r == c + 1 && j0 == (r & 7) && r < w) pivot(r);
     }
     __syncthreads();
   }
