@@ -155,7 +155,9 @@ struct Step {
   int count = 0, total_tiles = 0, max_m = 0, max_n = 0;
   int k0 = 0, nb = 0, blocked = 0;
   bool preload = false;  // GEMM: accumulators start from Cin (all problems alpha, beta = +-1)
-  int form = 0;          // GEMM: 1 four real products, 4 Gauss-Jordan update, 5 / 6 3M (zgemm_choose_form); OZ_MMA: digit pairs (34 or 28)
+  // GEMM: 1 four real products, 4 Gauss-Jordan update, 5 / 6 3M (zgemm_choose_form);
+  // OZ_MMA: digit pairs (34 or 28)
+  int form = 0;
   int uniform_tiles = 0; // GEMM: tiles of every problem when all have the same count, else 0
   size_t smem = 0;
   double flops = 0.0;    // real flops of the step (8mnk per complex GEMM)
@@ -337,8 +339,9 @@ struct GnUpward {
 void build_rgf_upward(Plan& plan, const std::vector<TriSystem>& sys, std::vector<RgfWork>& work,
                       GnUpward* gn = nullptr);
 // Downward pass (src/matinvertndiag_rgf.jl:166-182) writing the tridiagonal of
-// M^{-1} (blocks below the diagonal whose output is null are not computed); with full_rows/full_cols the whole inverse (rgf.jl:185-199) is
-// written into full[s][i*npl+j] (null = skip).
+// M^{-1} (blocks below the diagonal whose output is null are not computed); with
+// full_rows/full_cols the whole inverse (rgf.jl:185-199) is written into
+// full[s][i*npl+j] (null = skip).
 // on_final(i), when given, is called once layer i's diagonal output is final
 // for every system (in layer order).
 void build_rgf_downward(Plan& plan, const std::vector<TriSystem>& sys, std::vector<RgfWork>& work,

@@ -121,7 +121,9 @@ bool make_partition(int npl, int d1, Partition& P) {
 // the level costs max(work, serial) + 0.1 min(work, serial).  The Schur
 // complement (T layers) is solved by the next level or by sequential RGF,
 // 7 steps per layer.  Levels are chosen by a memoised search over layer counts
-// (interior sizes up to 256, at most max_levels levels).
+// (interior sizes up to 256, at most max_levels levels).  The constants were fitted
+// to launches of 8 us; chained ones of small blocks take about 5.5, and three to
+// five per layer instead of seven.
 struct GpuCost {
   double gemm_s, step_s;
   int nsys;

@@ -72,12 +72,12 @@ __device__ __forceinline__ unsigned gj_key(double v, int row) {
 //    the slab take the rank-8 update on the FP64 tensor path (16 x 8 tiles, k =
 //    8, four real products): W += S Bb, and W = S Bb at the pivot rows (the
 //    form W += (S - E_P) Bb would lose digits where |S| is far below 1).
-// What bounds it: the latency of a column (750 cycles with one warp of rows, 830
-// with four, 1040 with eight: two reduction rounds, a barrier of the warps with
+// What bounds it: the latency of a column (690 cycles with one warp of rows, 800
+// with four, 980 with eight: two reduction rounds, a barrier of the warps with
 // rows, one reciprocal, and some 250 instructions per warp) and the FP64 pipe of
 // one SM in the rank-8 updates.  Eight columns keep a row in 32 registers; wider
 // sub-panels do more of the n w^2 work in the latency-bound form, narrower ones
-// add update passes over shared memory.  A 256 x 32 panel takes 40 us (104 us
+// add update passes over shared memory.  A 256 x 32 panel takes 35 us (104 us
 // with the whole slab in registers and one rank-1 step per column).
 template <int T, int RT>
 __global__ void __launch_bounds__(T, 1)
@@ -345,10 +345,10 @@ __global__ void __launch_bounds__(T, 1)
 // scheduler partitions (warp mod 4): FP64 tensor instructions of a warp beside
 // them would delay every step of the column loop.  Odd CTAs take the opposite
 // partitions, so that CTAs that share an SM spread over all of them.
-// Bound: the latency of the column loop (750 to 1000 cycles a column) up to n =
+// Bound: the latency of the column loop (690 to 950 cycles a column) up to n =
 // 64, the FP64 pipes of one SM above.  Against one sub-panel and one update after
-// the other: one matrix of 50: 33 us (42), of 64: 38 (52), 592 of them 110 (124);
-// 512 of 32: 25 (41); one of 100: 108 (111), 296 of them 216 (224).  Two
+// the other: one matrix of 50: 30 us (42), of 64: 36 (52), 592 of them 112 (124);
+// 512 of 32: 24 (41); one of 100: 106 (111), 296 of them 217 (224).  Two
 // factoring warps with two rows per thread take 7 % longer at 100.
 template <int T>
 __global__ void __launch_bounds__(T, 512 / T) zgj_whole_kernel(const ZInvProblem* __restrict__ probs) {

@@ -18,8 +18,9 @@
 // Without row interchanges (the selected inverse of NEGF matrices) no panel of
 // whole columns is needed: a kernel factors a 32 x 32 diagonal block and inverts
 // its triangles, a second one substitutes A21 U^{-1} and L^{-1} A12, and the
-// engine forms the Schur update as a product.  Triangular inverse: diagonal blocks of 32 inverted in shared
-// memory here, then pairs of blocks joined by products, doubling their size.
+// engine forms the Schur update as a product.  Triangular inverse: diagonal blocks
+// of 32 inverted in shared memory here, then pairs of blocks joined by products to
+// 64, then block columns of that width.
 #include "negf_common.cuh"
 
 namespace negf {

@@ -30,7 +30,7 @@ def _dev(rng, npl, b):
     return negf.Device(Hd, Hu, s, s), M
 
 
-@pytest.mark.parametrize("npl,b", [(12, 5), (8, 40), (4, 112), (4, 144), (3, 272)])
+@pytest.mark.parametrize("npl,b", [(1, 30), (2, 33), (12, 5), (8, 40), (4, 112), (4, 144), (3, 272)])
 def test_keldysh(negf, npl, b):
     """G S G^H on the block tridiagonal; bound: n u cond(M) for each factor G."""
     rng = np.random.default_rng(npl * b)
